@@ -113,6 +113,8 @@ _SIGNATURES = {
     "fennol_mlp_workspace_bytes": (SZ, [I, I, I, C.POINTER(MLPWeights)]),
     "fennol_mlp_energy_grad": (I, [I, I, I, P, P, C.POINTER(MLPWeights), P, P, P, P, P, SZ, P]),
     "fennol_mlp_energy_grad_active": (I, [I, I, I, P, P, C.POINTER(MLPWeights), P, P, ULL, P, P, P, SZ, P]),
+    "fennol_mlp_energy_grad_groups": (I, [I, I, I, P, P, C.POINTER(MLPWeights), P, P, P, P, I, P, P, P, SZ, P]),
+    "fennol_aev_active_groups": (I, [C.POINTER(AEVParams), C.c_uint, P, I]),
     "fennol_aev_active_chunks": (ULL, [C.POINTER(AEVParams), C.c_uint]),
     "fennol_energy_workspace_bytes": (SZ, [I, I]),
     "fennol_energy_reduce": (I, [P, P, I, P, I, D, P, P, P, SZ, P]),

@@ -217,6 +217,7 @@ int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_
                                                        m == 0, e_rows);
       if (cudaGetLastError() != cudaSuccess) return FENNOL_ERR_CUDA;
     }
+    if (!dx) continue;  // energies only
     // backward layers 3..2: G_{l} = (G_{l+1} W_{l+1}^T) * celu'(H_l), in place of H_l
     for (int l = 2; l >= 1; --l) {
       GemmArgs a{};

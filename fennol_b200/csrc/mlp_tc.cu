@@ -459,19 +459,19 @@ size_t fnl_mlp_tc_workspace(int precision, int rows, int n_models, const fennol_
   (void)n_models;
   size_t a = tc_layout(rows, w, nullptr, nullptr);
   if (fnl_mlp_fused_supported(precision, w)) {
-    size_t b = fnl_mlp_fused_workspace(w);
+    size_t b = fnl_mlp_fused_workspace(rows, w);
     if (b > a) a = b;
   }
   return a;
 }
 
 int fnl_mlp_tc(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
-               const fennol_mlp_weights* w, const void* x, const void* x_lo, unsigned long long kmask,
+               const fennol_mlp_weights* w, const void* x, const void* x_lo, ColumnGroups xg, ColumnGroups dg,
                float* e_rows, float* dx, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (!encode_fn()) return FENNOL_ERR_UNSUPPORTED;
   const bool f16 = precision == FENNOL_MLP_F16X3X1 || precision == FENNOL_MLP_F16X3X2;
   if (fnl_mlp_fused_supported(precision, w) && (f16 || !getenv("FENNOL_MLP_UNFUSED")))
-    return fnl_mlp_fused(precision, rows, ntiles, tile_species, tile_row, w, x, x_lo, kmask, e_rows, dx, ws,
+    return fnl_mlp_fused(precision, rows, ntiles, tile_species, tile_row, w, x, x_lo, xg, dg, e_rows, dx, ws,
                          ws_bytes, st);
   if (f16) return FENNOL_ERR_UNSUPPORTED;  // the FP16 forms exist only as the fused kernel
   const int* d = w->dims;
@@ -546,6 +546,7 @@ int fnl_mlp_tc(int precision, int rows, int ntiles, const int* tile_species, con
     g.p.rows = rows;
     g.p.first_model = m == 0;
     if ((rc = launch(g, rows, ntiles, st))) return rc;
+    if (!dx) continue;  // energies only
     // B3: G2 = (G3 W3^T) * celu'(H2), in place of H2
     g = base(EPI_DACT, t.g3, t.g3l, d[3], w->w_hi[2], w->w_lo[2], d[2], d[2], d[2] / 2, g0);
     g.p.act_hi = t.h2;

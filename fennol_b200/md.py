@@ -208,7 +208,7 @@ class MDEngine:
         if self.trigger == "displacement":
             n += 1
         n += 1 if self.skin > 0 else 0
-        n += 1 + self.pot.mlp_launches() + 1 + 1  # aev fwd, mlp, energy sum, aev bwd
+        n += 1 + self.pot.mlp_launches(self.layout.ntiles) + 1 + 1  # aev fwd, mlp, energy sum, aev bwd
         return n
 
     def rebuild_launches(self) -> int:

@@ -438,6 +438,7 @@ class ANIPotential:
         self.minimum_image = minimum_image
         self._cache: Dict[tuple, tuple] = {}
         self._chunk_masks: Dict[int, int] = {}
+        self._group_masks: Dict[int, np.ndarray] = {}
         self.capacity_margin = 1.05
         self.add_neigh = 8
         # repeated calls on the same batch replay one captured CUDA graph
@@ -487,18 +488,33 @@ class ANIPotential:
             self._chunk_masks[species_mask] = m
         return m
 
-    def mlp_launches(self) -> int:
-        """Kernels launched by one fennol_mlp_energy_grad call: the FP32 form
-        runs 7 per model, the fused tcgen05 kernel (BF16 / BF16x2 on these
-        layer sizes) one, the unfused tcgen05 path 6 per model and one sum."""
+    def active_groups(self, species_mask: int) -> np.ndarray:
+        """The 16-column groups of the AEV rows that can be non-zero for a
+        batch of these species (``fennol_aev_active_groups``), as mask words."""
+        words = self._group_masks.get(species_mask)
+        if words is None:
+            words = np.zeros(_ceil(self.mlp.dims[0], 1024) // 1024, np.uint64)
+            call("fennol_aev_active_groups", C_ptr(self.params), species_mask, words.ctypes.data, words.size)
+            self._group_masks[species_mask] = words
+        return words
+
+    def mlp_launches(self, ntiles: Optional[int] = None) -> int:
+        """Kernels launched by one MLP call: the FP32 form runs 7 per model,
+        the fused tcgen05 kernel (BF16 / BF16x2 on these layer sizes and the
+        FP16 forms) one, and one more for an ensemble on ``ntiles`` row tiles
+        that its CTAs share; the unfused tcgen05 path 6 per model and one sum."""
         import os
         if self.precision == _lib.MLP_FP32:
             return 7 * self.mlp.n_models
-        if self.precision in _lib.F16_FORMS:
+        fused = self.precision in _lib.F16_FORMS or (
+            self.precision in (_lib.MLP_BF16, _lib.MLP_BF16X2) and self.mlp.dims[0] % 256 == 0
+            and max(self.mlp.dims[1:4]) <= 256 and not os.environ.get("FENNOL_MLP_UNFUSED"))
+        if not fused:
+            return 6 * self.mlp.n_models + 1
+        if not ntiles or self.mlp.n_models == 1:
             return 1
-        fused = (self.precision in (_lib.MLP_BF16, _lib.MLP_BF16X2) and self.mlp.dims[0] % 256 == 0
-                 and max(self.mlp.dims[1:4]) <= 256 and not os.environ.get("FENNOL_MLP_UNFUSED"))
-        return 1 if fused else 6 * self.mlp.n_models + 1
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        return 2 if ntiles % min(sms, ntiles * self.mlp.n_models) else 1
 
     # --------------------------------------------------------------- launches
     def launch_forces(self, layout: BatchLayout, g: GraphBuffers, ws: Workspace, stream: int,
@@ -526,13 +542,17 @@ class ANIPotential:
                  layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
                  g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.aev_kind, ws.x.data_ptr(),
                  _ptr(ws.x_lo), ws.x.shape[1], ws.status.data_ptr(), stream)
-        call("fennol_mlp_energy_grad_active", self.precision, layout.rows, layout.ntiles,
+        # the columns that can be non-zero are also the ones the adjoint reads
+        groups = self.active_groups(layout.species_mask)
+        call("fennol_mlp_energy_grad_groups", self.precision, layout.rows, layout.ntiles,
              layout.t_tile_species.data_ptr(), layout.t_tile_row.data_ptr(), C_ptr(self.mlp.struct),
-             ws.x.data_ptr(), _ptr(ws.x_lo), self.active_chunks(layout.species_mask), ws.e_rows.data_ptr(),
-             ws.dx.data_ptr(), ws.mlp_ws.data_ptr(), ws.mlp_ws.numel(), stream)
+             ws.x.data_ptr(), _ptr(ws.x_lo), groups.ctypes.data, groups.ctypes.data, groups.size,
+             ws.e_rows.data_ptr(), ws.dx.data_ptr() if want_forces else None, ws.mlp_ws.data_ptr(),
+             ws.mlp_ws.numel(), stream)
         if ghost_rows is not None and ghost_rows.numel() > 0:
             ws.e_rows.index_fill_(0, ghost_rows, 0.0)
-            ws.dx.index_fill_(0, ghost_rows, 0.0)
+            if want_forces:
+                ws.dx.index_fill_(0, ghost_rows, 0.0)
         call("fennol_energy_reduce", ws.e_rows.data_ptr(), layout.t_atom_row.data_ptr(), n,
              layout.t_sys_start.data_ptr(), layout.nsys, float(self.unit_scale), ws.energy.data_ptr(),
              ws.e_atom.data_ptr(), ws.energy_ws.data_ptr(), ws.energy_ws.numel(), stream)

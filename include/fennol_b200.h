@@ -189,6 +189,16 @@ int fennol_aev_length(const fennol_aev_params* p);
 unsigned long long fennol_aev_active_chunks(const fennol_aev_params* p, unsigned species_mask);
 
 /*
+ * Host only.  The same in groups of 16 columns, the widths of the radial and
+ * angular blocks being multiples of 16: bit g % 64 of host_groups[g / 64]
+ * covers columns [16g, 16g + 16).  Writes every one of the `words` words and
+ * returns the number of groups named, or FENNOL_ERR_INVALID when `words` do
+ * not hold the row, FENNOL_ERR_UNSUPPORTED for unsupported parameters.
+ */
+int fennol_aev_active_groups(const fennol_aev_params* p, unsigned species_mask,
+                             unsigned long long* host_groups, int words);
+
+/*
  * Pack positions and species for the AEV kernels: xyzs[i] = (x, y, z,
  * species index as int bits).  species_idx are positions in species_order.
  */
@@ -374,6 +384,28 @@ int fennol_mlp_energy_grad_active(int precision, int rows, int ntiles, const int
                                   const int* tile_row, const fennol_mlp_weights* w, const void* x,
                                   const void* x_lo, unsigned long long active_chunks, float* e_rows,
                                   float* dx, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * The same with the columns named in groups of 16 and the two sides apart: bit
+ * g % 64 of word g / 64 stands for columns [16 g, 16 g + 16).
+ *   host_x_groups (host memory; NULL: all): the columns of x that may be
+ *     non-zero.  The caller guarantees that every other column is zero in
+ *     every row, and its products may be left out of the first layer.
+ *   host_dx_groups (host memory; NULL: all): the columns of dx that are
+ *     wanted.  The fused tensor-core forms leave the other columns of dx as
+ *     they were, the other forms may write them.
+ *   group_words: words of each array given, at least dims[0] / 1024 rounded
+ *     up, else FENNOL_ERR_INVALID (as are x groups that name no column, for
+ *     the fused forms).
+ *   dx NULL: energies only, without the input-gradient GEMMs.
+ * For AEV rows, fennol_aev_active_groups gives the groups of a species set.
+ */
+int fennol_mlp_energy_grad_groups(int precision, int rows, int ntiles, const int* tile_species,
+                                  const int* tile_row, const fennol_mlp_weights* w, const void* x,
+                                  const void* x_lo, const unsigned long long* host_x_groups,
+                                  const unsigned long long* host_dx_groups, int group_words,
+                                  float* e_rows, float* dx, void* workspace, size_t workspace_bytes,
+                                  void* stream);
 
 /*
  * Failure handling of the fused tensor-core MLP (no counterpart in the

@@ -201,3 +201,90 @@ def test_active_chunks_match_dense(cuda_device, precision):
     np.testing.assert_allclose(da[:, cols], dd[:, cols], rtol=1e-5, atol=1e-7 * np.abs(dd).max())
     inactive = np.setdiff1d(np.arange(da.shape[1]), cols)
     assert not da[:, inactive].any()   # never written
+
+
+def _row_results(pot, layout, ws, x_groups, dx_groups, want_dx=True):
+    """Row energies and dE/dAEV of one MLP call on the workspace's AEV rows,
+    into buffers filled with a marker."""
+    from fennol_b200._lib import call
+    from fennol_b200.potential import C_ptr, _ptr
+
+    e_rows = torch.full_like(ws.e_rows, 7.0)
+    dx = torch.full_like(ws.dx, 7.0)
+    words = max(len(x_groups) if x_groups is not None else 0, len(dx_groups) if dx_groups is not None else 0)
+    call("fennol_mlp_energy_grad_groups", pot.precision, layout.rows, layout.ntiles,
+         layout.t_tile_species.data_ptr(), layout.t_tile_row.data_ptr(), C_ptr(pot.mlp.struct), ws.x.data_ptr(),
+         _ptr(ws.x_lo), None if x_groups is None else x_groups.ctypes.data,
+         None if dx_groups is None else dx_groups.ctypes.data, words, e_rows.data_ptr(),
+         dx.data_ptr() if want_dx else None, ws.mlp_ws.data_ptr(), ws.mlp_ws.numel(),
+         torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    if pot.precision != 0:
+        assert _err_word(pot) == 0
+    return e_rows.cpu().numpy(), dx.cpu().numpy()
+
+
+def _columns(groups):
+    return np.array([c for g in range(64 * len(groups)) if (int(groups[g // 64]) >> (g % 64)) & 1
+                     for c in range(16 * g, 16 * g + 16)])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16", "bf16x2", "f16x3x1", "f16x3x2", "bf16x3"])
+@pytest.mark.parametrize("molecules", [False, True])
+def test_column_groups_match_dense(cuda_device, precision, molecules):
+    """The column groups of a species set, the energies-only call and odd sets
+    of wanted columns give the dense call's values bit for bit: the columns
+    left out are zero in every row, and the order of the other products is the
+    same.  The fused forms leave columns that are not wanted as they were."""
+    pot = ANIPotential(precision=precision, device=cuda_device, seed=0, n_models=2)
+    if molecules:
+        mols = molecule_batch(5, seed=11)
+        xyz, sp = np.concatenate([m.coordinates for m in mols]), np.concatenate([m.species for m in mols])
+        pot.energy_and_forces(xyz, sp, [m.natoms for m in mols])
+    else:
+        s = water_box(4, seed=2)
+        pot.energy_and_forces(s.coordinates, s.species, [s.natoms], s.cell[None])
+    layout, g, ws = next(iter(pot._cache.values()))
+    groups = pot.active_groups(layout.species_mask)
+    ws.x[:, pot.aev_cfg.aev_length:] = 0
+    e, dx = _row_results(pot, layout, ws, None, None)
+    odd = groups.copy()
+    odd[0] &= np.uint64(0xF7FF_FFFF_FBFF_FFFB)  # leaves some out: runs of every length
+    for want in (groups, odd):
+        e2, dx2 = _row_results(pot, layout, ws, groups, want)
+        assert np.array_equal(e2, e)
+        cols = _columns(want)
+        assert np.array_equal(dx2[:, cols], dx[:, cols])
+        if precision not in ("fp32", "bf16x3"):
+            assert (dx2[:, np.setdiff1d(np.arange(dx.shape[1]), cols)] == 7.0).all()
+    e3, dx3 = _row_results(pot, layout, ws, groups, None, want_dx=False)
+    assert np.array_equal(e3, e) and (dx3 == 7.0).all()
+
+
+@pytest.mark.parametrize("n_side,n_models", [(4, 3), (9, 8), (19, 2), (21, 3)])
+def test_shared_tiles_are_the_mean_of_the_models(cuda_device, n_side, n_models):
+    """Ensembles whose (tile, model) items the CTAs share out inside tiles
+    (fewer items than SMs, some per CTA, many per CTA with a ragged end): the
+    row energies and dE/dAEV are the mean of the single-model results.
+    float32 sums of at most eight models: 8 half-ulps of the largest term."""
+    W = init_weights(CFG, MCFG, seed=3, n_models=n_models)
+    s = water_box(n_side, seed=n_side)
+    pot = ANIPotential(precision="f16x3x1", device=cuda_device, weights=W)
+    pot.energy_and_forces(s.coordinates, s.species, [s.natoms], s.cell[None])
+    layout, g, ws = next(iter(pot._cache.values()))
+    groups = pot.active_groups(layout.species_mask)
+    e, dx = _row_results(pot, layout, ws, groups, groups)
+    cols = _columns(groups)
+    es, ds = [], []
+    for m in range(n_models):
+        one = ANIPotential(precision="f16x3x1", device=cuda_device, weights=[W[m]])
+        one.energy_and_forces(s.coordinates, s.species, [s.natoms], s.cell[None])
+        lay1, _, ws1 = next(iter(one._cache.values()))
+        e1, d1 = _row_results(one, lay1, ws1, groups, groups)
+        es.append(e1.astype(np.float64))
+        ds.append(d1[:, cols].astype(np.float64))
+    used = np.concatenate([np.arange(r, r + 128) for r in layout.t_tile_row.cpu().numpy()])
+    tol = 8 * 2.0 ** -24
+    em, dm = np.mean(es, 0)[used], np.mean(ds, 0)[used]
+    assert np.abs(e[used] - em).max() <= tol * np.abs(es).max()
+    assert np.abs(dx[used][:, cols] - dm).max() <= tol * np.abs(ds).max()
