@@ -44,7 +44,7 @@ int energy_grad(int precision, int rows, int ntiles, const int* tile_species, co
     return FENNOL_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   if (precision == FENNOL_MLP_FP32)
-    return fnl_mlp_simt(rows, ntiles, tile_species, tile_row, w, (const float*)x, e_rows, dx, workspace, st);
+    return fnl_mlp_simt(rows, ntiles, tile_species, tile_row, w, (const float*)x, xg, dg, e_rows, dx, workspace, st);
   if (precision != FENNOL_MLP_BF16 && !x_lo) return FENNOL_ERR_INVALID;
   return fnl_mlp_tc(precision, rows, ntiles, tile_species, tile_row, w, x, x_lo, xg, dg, e_rows, dx, workspace,
                     workspace_bytes, st);

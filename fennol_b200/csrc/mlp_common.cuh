@@ -28,8 +28,8 @@ struct ColumnGroups {
 // NULL: energies only.
 size_t fnl_mlp_simt_workspace(int rows, const fennol_mlp_weights* w);
 int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_row,
-                 const fennol_mlp_weights* w, const float* x, float* e_rows, float* dx, void* ws,
-                 cudaStream_t st);
+                 const fennol_mlp_weights* w, const float* x, fnl::ColumnGroups xg, fnl::ColumnGroups dg,
+                 float* e_rows, float* dx, void* ws, cudaStream_t st);
 size_t fnl_mlp_tc_workspace(int precision, int rows, int n_models, const fennol_mlp_weights* w);
 int fnl_mlp_tc(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
                const fennol_mlp_weights* w, const void* x, const void* x_lo, fnl::ColumnGroups xg,

@@ -499,13 +499,14 @@ class ANIPotential:
         return words
 
     def mlp_launches(self, ntiles: Optional[int] = None) -> int:
-        """Kernels launched by one MLP call: the FP32 form runs 7 per model,
-        the fused tcgen05 kernel (BF16 / BF16x2 on these layer sizes and the
+        """Kernels launched by one MLP call: the FP32 form runs 7 per
+        model, or per several models on few ``ntiles`` row tiles; the fused tcgen05 kernel (BF16 / BF16x2 on these layer sizes and the
         FP16 forms) one, and one more for an ensemble on ``ntiles`` row tiles
         that its CTAs share; the unfused tcgen05 path 6 per model and one sum."""
         import os
         if self.precision == _lib.MLP_FP32:
-            return 7 * self.mlp.n_models
+            per = 1 if not ntiles else min(self.mlp.n_models, max(1, 2400 // (3 * ntiles)))
+            return 7 * -(-self.mlp.n_models // per)
         fused = self.precision in _lib.F16_FORMS or (
             self.precision in (_lib.MLP_BF16, _lib.MLP_BF16X2) and self.mlp.dims[0] % 256 == 0
             and max(self.mlp.dims[1:4]) <= 256 and not os.environ.get("FENNOL_MLP_UNFUSED"))

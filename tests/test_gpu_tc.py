@@ -288,3 +288,32 @@ def test_shared_tiles_are_the_mean_of_the_models(cuda_device, n_side, n_models):
     em, dm = np.mean(es, 0)[used], np.mean(ds, 0)[used]
     assert np.abs(e[used] - em).max() <= tol * np.abs(es).max()
     assert np.abs(dx[used][:, cols] - dm).max() <= tol * np.abs(ds).max()
+
+
+@pytest.mark.parametrize("groups", [False, True])
+def test_fp32_form_takes_buffers_off_16_bytes(cuda_device, groups):
+    """The FP32 form reads four floats at a time only where every array is
+    16-byte aligned; on rows and gradients that start one float further on it
+    gives the same bits."""
+    from fennol_b200._lib import call
+    from fennol_b200.potential import C_ptr
+
+    pot = ANIPotential(precision="fp32", device=cuda_device, seed=0, n_models=3)
+    s = water_box(4, seed=2)
+    pot.energy_and_forces(s.coordinates, s.species, [s.natoms], s.cell[None])
+    layout, g, ws = next(iter(pot._cache.values()))
+    words = pot.active_groups(layout.species_mask)
+    got = []
+    for off in (0, 1):
+        x = torch.zeros(ws.x.numel() + 1, device=cuda_device)
+        x[off:off + ws.x.numel()] = ws.x.flatten()
+        dx = torch.zeros(ws.x.numel() + 1, device=cuda_device)
+        e_rows = torch.zeros_like(ws.e_rows)
+        call("fennol_mlp_energy_grad_groups", pot.precision, layout.rows, layout.ntiles,
+             layout.t_tile_species.data_ptr(), layout.t_tile_row.data_ptr(), C_ptr(pot.mlp.struct),
+             x.data_ptr() + 4 * off, None, words.ctypes.data if groups else None,
+             words.ctypes.data if groups else None, len(words), e_rows.data_ptr(), dx.data_ptr() + 4 * off,
+             ws.mlp_ws.data_ptr(), ws.mlp_ws.numel(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        got.append((e_rows.cpu().numpy(), dx[off:off + ws.x.numel()].cpu().numpy()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
