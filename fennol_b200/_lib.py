@@ -126,6 +126,8 @@ _SIGNATURES = {
     "fennol_check_finite": (I, [I, P, P, P, P, P]),
     "fennol_net_loss_grad_workspace_bytes": (SZ, [C.POINTER(NetTrain), P]),
     "fennol_net_loss_grad": (I, [C.POINTER(NetTrain), P, P, P, P, I, P, P, SZ, P]),
+    "fennol_loss_seed_workspace_bytes": (SZ, [I]),
+    "fennol_loss_seed": (I, [P, P, I, P, P, I, P, P, D, D, P, P, P, I, P, P, SZ, P]),
     "fennol_mlp_wait_limit": (I, [D]),
     "fennol_mlp_inject_stall": (I, [I]),
     "fennol_capture_if_begin": (I, [P, P, P]),

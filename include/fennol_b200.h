@@ -466,6 +466,25 @@ int fennol_net_loss_grad(const fennol_net_train* net, const int* host_row0, cons
                          const void* x, const void* t, int ld, const void* c_row, void* workspace,
                          size_t workspace_bytes, void* stream);
 
+/* Workspace of fennol_loss_seed, in bytes. */
+size_t fennol_loss_seed_workspace_bytes(int natoms);
+
+/*
+ * The loss L = w_e mean_b (E_b - e_ref_b)^2 + w_f mean (F - f_ref)^2 of
+ * FeNNol's training (training/utils.py:140-525) and its seeds, in two launches:
+ *   du4[natoms*4]: (dL/dF of each atom, 0), the displacement field of
+ *     fennol_aev_tangent (float32);
+ *   c_row[atom_row[i]] = dL/dE of atom i's system (float32, float64 when
+ *     is_double), the row seeds of fennol_net_loss_grad;
+ *   terms[FENNOL_STATUS_WORDS + 2]: the status words at that point of the
+ *     stream as float64, then the energy and the force term.
+ * energy, e_ref [nsys] and f_ref [natoms*3] are float64, forces float32.
+ */
+int fennol_loss_seed(const double* energy, const double* e_ref, int nsys, const float* forces,
+                     const double* f_ref, int natoms, const int* atom_sys, const int* atom_row, double w_e,
+                     double w_f, const int* status, float* du4, void* c_row, int is_double, double* terms,
+                     void* workspace, size_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Reductions and outputs                                                    */
 /* ------------------------------------------------------------------------ */
