@@ -6,26 +6,28 @@
 // model) items and runs, for each, the six GEMMs of the layer chain
 //     L1 X.W1  L2 H1.W2  L3 H2.W3 (+ energy head)  B3 G3.W3^T  B2 G2.W2^T  B1 G1.W1^T
 // (energies only: the first three) keeping the activations on chip:
-//   * warp 0 (one thread) streams the AEV tile and W1^T through an L1 ring laid
-//     over the activation buffer and the weight slots, then all other weights
-//     through the weight slots;
-//   * warp 1 owns the 512 TMEM columns (two 256-column FP32 accumulators used
-//     alternately) and one thread issues tcgen05.mma / tcgen05.commit;
+//   * warp 0 streams the AEV tile and all weights through one TMA ring in shared
+//     memory, in the order the GEMMs take them, as far ahead as the ring holds;
+//   * warp 1 owns the 512 TMEM columns (two regions of 256, accumulators and
+//     activations in turn) and issues tcgen05.mma / tcgen05.commit;
 //   * warps 2-17 are the epilogue: they read an accumulator (tcgen05.ld, one
 //     row per thread, four warps per lane quarter), apply bias + CELU, the
-//     energy head, or CELU' masks, and write the next A operand as 16-bit hi
-//     (+ lo) pairs straight into shared memory in the 128-byte-swizzled K-major
-//     layout the MMA descriptors expect (fence.proxy.async before the MMA
-//     reads it).
-// What bounds it: the chain of GEMM -> epilogue -> GEMM of one item, which
-// nothing else fills.  So the epilogue is short (packed FP32 instructions, no
-// selects, biases in shared memory, no spills: with 16 warps a spilled register
-// is an L2 round trip, 62k cycles per water item against 47k), its warps finish
-// one 64-column K-atom after the other so that the next GEMM starts early, and
-// dX is summed over the models in scratch instead of by bulk adds, which held
-// up the loads of the next item.  98,304 atoms x 8 models (f16x3x1, water):
-// 1.53 ms with 8 epilogue warps, 64-column chunks and whole tiles per CTA,
-// 0.97 ms now; 192 atoms x 8 models 0.25 ms to 0.035 ms.
+//     energy head, or CELU' masks, and put the next A operand, 16-bit hi (+ lo)
+//     pairs, over it in tensor memory (tcgen05.st).
+// What bounds it: the chain of GEMM -> epilogue -> GEMM of one item, about 36k
+// cycles for a water tile, of which the MMAs are 15k and the streaming of 0.96
+// MB of operands at 50 bytes per cycle 19k; neither is full, each waits for the
+// other at the ends of a GEMM.  So the epilogue is short (packed FP32
+// instructions, no selects, biases in shared memory, no spills: with 16 warps a
+// spilled register is an L2 round trip), its warps finish one 64-column K-atom
+// after the other so that the next GEMM starts early, dX is summed over the
+// models in scratch (bulk adds held up the loads of the next item), and the
+// activations stay in tensor memory: through shared memory, the A operand's
+// reads and writes and the W chunks took its whole bandwidth in L2 and L3, and
+// the ring was too small to prefetch the next item.  98,304 atoms x 8 models
+// (f16x3x1, water): 1.53 ms at first (62k cycles an item, whole tiles per CTA),
+// 0.97 ms with the activations in shared memory (47k), 0.85 ms now; 192 atoms x 8
+// models 0.25 ms at first, 0.03 ms now.
 // Operand forms: BF16 (A hi, optionally A lo; weights BF16) and FP16 (the
 // kernel template's F16 flag).  The FP16 forms split the activations and the
 // power-of-two-scaled float32 weights into float16 hi + lo: the forward GEMMs
@@ -36,15 +38,18 @@
 // Active columns: the caller names the 16-column groups (one MMA K step each)
 // of the input that may be non-zero; L1 leaves the K steps of the others out
 // (their products are zero: the sums do not change) and streams only units of
-// 64 or 32 columns that hold one.  B1 computes dX for the groups asked for, in
-// runs of up to 16, whatever lies between them.
+// 32 columns that hold one.  B1 computes dX for the groups asked for, in runs of
+// up to 8, whatever lies between them.
 // CELU' of layers 1-2 (needed by the backward) goes to a per-CTA scratch in
-// global memory that stays L2 resident.  The models of a tile are summed in
-// model order, those of a tile shared by CTAs part by part, so the per-row
-// energy and dE/dAEV sums are deterministic.  Every wait is bounded (2 s); a timeout sets the error word,
-// raises a shared abort flag that ends all roles, and the CTA frees its TMEM.
+// global memory that stays L2 resident.  Row energies are summed in model order,
+// and so is dE/dAEV (in tiles that CTAs share only up to 16 column groups, else
+// part by part), always in the same way for the same batch.  Every wait is
+// bounded (2 s); a timeout sets the error word, raises a shared abort flag that
+// ends all roles, and the CTA frees its TMEM.
 #include <cuda.h>
 #include <cudaTypedefs.h>
+
+#include <algorithm>
 
 #include "mlp_common.cuh"
 #include "umma.cuh"
@@ -58,28 +63,22 @@ constexpr int kEpiWarps = 16;                     // four per TMEM lane quadrant
 constexpr int kThreads = (2 + kEpiWarps) * 32;
 constexpr int BM = 128, BK = 64;
 constexpr int kGroup = 16;                        // columns of one active-column group: one MMA K step
-constexpr uint32_t kAtom = BM * BK * 2;           // one 128 x 64 16-bit K-atom: 16 KB
-constexpr uint32_t kActHalf = 4 * kAtom;          // up to K = 256 per hi (or lo) operand
-constexpr uint32_t kActBytes = 2 * kActHalf;      // 128 KB
-constexpr uint32_t kWStage = 256 * BK * 2;        // 32 KB
-// Operand memory: activations hi [0, 64 K), activations lo [64 K, 128 K),
-// weight slots 0 and 1 [128 K, 192 K).  Weight slots 2 and 3 are the lo half
-// of the activations: the input-gradient GEMMs of forms without gradient lo
-// parts leave it free once L3 has run.
-constexpr int kWSlots = 4;
-constexpr uint32_t kRing = kActBytes + 2 * kWStage;  // 192 KB
-// L1 ring: stages of one column unit (64 columns with 128-byte swizzle, or 32
-// with 64-byte swizzle), A hi | A lo | B hi (| B lo), laid through the operand
-// memory from 64 K on and round to its start, so that the first stages avoid
-// the activations hi, which the last GEMM of the previous item still reads.
-constexpr int kXStages = 6;
-constexpr uint32_t kXBase = kActHalf;
-constexpr int kMaxUnits = 4096 / 32, kMaxGroups = 4096 / kGroup;
-constexpr uint32_t kXpose = kEpiWarps * 32 * kGroup * 4;  // per-epilogue-warp 32 x 16 dX staging tiles: 32 KB
-constexpr uint32_t kSmemMain = kRing + kXpose;            // 224 KB
-// The same 32 KB hold an item's biases and last kernel (b1 | b2 | b3 | w4, 256
-// floats each) until its dX leaves.
+// Shared memory: a ring that every operand from global memory streams through
+// (activations live in tensor memory), an item's biases and last kernel (b1 | b2
+// | b3 | w4, 256 floats each), and per-epilogue-warp 32 x 16 dX staging tiles.
+// Ring components (an A or B tile of a chunk) start on 4 KB.
+constexpr uint32_t kRing = 46 * 4096;
 constexpr int kBias = 256;
+constexpr uint32_t kXpose = kEpiWarps * 32 * kGroup * 4;
+constexpr uint32_t kSmemMain = kRing + 4 * kBias * 4 + kXpose;
+constexpr int kChunks = 16;      // chunks in flight at most
+// L1 streams units of 32 columns (64-byte swizzle): half of a 64-column unit
+// would often be zero columns, and with all columns active two of those (96 KB
+// each with the W1 low parts) do not fit the ring: 256 molecules x 8 models 0.50
+// ms against 0.54, 98,304 atoms x 8, 8 MD steps 16.1 ms against 16.6.
+constexpr int kUnit = 32;
+constexpr int kMaxUnits = 4096 / kUnit, kMaxGroups = 4096 / kGroup;
+constexpr int kRunGroups = 8;    // dX column groups of one B1 run (128 columns)
 // bounded waits: default limit, and the settings of fennol_mlp_wait_limit /
 // fennol_mlp_inject_stall (host side)
 constexpr uint64_t kTimeoutNs = 2000000000ull;
@@ -91,17 +90,8 @@ struct FusedParams {
   const int* tile_species;
   const int* tile_row;
   int d0, d1, d2, d3;
-  int a_lo;   // forward A operands (X, H1, H2) carry a lo part
-  int g_lo;   // input-gradient A operands (G3, G2, G1) carry a lo part
-  int wf_lo;  // forward GEMMs add A_hi x W_lo
   int wb_lo;  // input-gradient GEMMs add G_hi x W_lo
-  int bslots;       // weight slots of the input-gradient GEMMs (4, or 2 with gradient lo parts)
-  int unit;         // columns of an L1 unit: 64 or 32
-  int nunits;       // active L1 units
-  int xstages;
-  uint32_t xstage;  // bytes of an L1 stage
-  uint32_t slot_stages[2];        // L1 stages that overlap weight slots 0, 1 (bit per stage)
-  uint32_t stage_slots[kXStages]; // weight slots that overlap an L1 stage (bits 0-3); bit 4: activations
+  int nunits;  // active L1 units
   float alpha, inv_models;
   unsigned long long timeout_ns;  // limit of every bounded wait
   int stall;                      // the load producer issues no copies (timeout tests)
@@ -114,54 +104,73 @@ struct FusedParams {
   float* e_rows;
   float* dx;
   float* dc;  // [gridDim.x][(d1 + d2) / 4][128][4]
-  // ensembles: dX summed over the models so far, [gridDim.x][2][d0 / 4][128][4]
-  // (first and other tiles of a CTA), and the energies of the models of tiles
-  // shared by CTAs, [ntiles][n_models][128]
+  // ensembles: dX summed over the models so far and dX of shared tiles,
+  // [gridDim.x][slots][ndx * 4][128][4], and the energies of the models of
+  // shared tiles, [tiles][n_models][128]
   float* xs;
   float* e_part;
+  int xs_slots;
+  int apart;  // the models of shared tiles have a slot each (else the parts of tiles)
   int* err;
   int ndx;                        // dX column groups (0: energies only)
   unsigned char xunit[kMaxUnits];   // L1 units and the K steps of each that are active (bit per 16 columns)
   unsigned char xbits[kMaxUnits];
   unsigned char dgroup[kMaxGroups]; // dX column groups, ascending
+  // the boxes that W1 rows of the groups are loaded in, run by run: first group, groups
+  unsigned char box_g[kMaxGroups], box_n[kMaxGroups];
 };
 
 struct Maps {
-  CUtensorMap x, xlo, w1t, w2t, w3t, w3, w2, w1, w1g;
-  CUtensorMap w1t_lo, w2t_lo, w3t_lo, w3_lo, w2_lo, w1_lo, w1g_lo;  // low parts (unused maps alias the high ones)
+  CUtensorMap x, xlo, w1t, w2t, w3t, w3, w2, w1, w1p, w1g;
+  CUtensorMap w1t_lo, w2t_lo, w3t_lo, w3_lo, w2_lo, w1_lo, w1p_lo, w1g_lo;  // low parts (unused maps alias the high ones)
   CUtensorMap dx;  // FP32 [rows][d0], 32-row x 16-column boxes, 64-byte swizzle
 };
 
-// The (tile, model) items of one CTA.  All items are numbered tile by tile and
-// cut into `blocks` contiguous ranges of (nearly) equal length, so a range may
-// begin and end inside a tile: those parts of a tile leave their sums in the
-// CTA's scratch and k_mlp_join adds the parts up in model order.  (Whole tiles
-// per CTA left 98,304 atoms x 8 models 6 tiles on some CTAs and 5 on others,
-// 12,288 atoms 52 of 148 SMs idle, and ran a small box's 8 models one after
-// the other.)
-__host__ __device__ __forceinline__ int first_item(int ntiles, int M, int block, int blocks) {
-  return (int)((long long)ntiles * M * block / blocks);
-}
+// The (tile, model) items of one CTA: `whole` tiles with all their models, then
+// a contiguous range (nearly equal ones) of the items of the tiles left over,
+// which CTAs share: they leave their dX in scratch and k_mlp_join adds the
+// models up.  (Whole tiles only gave 98,304 atoms x 8 models 6 tiles on some
+// CTAs and 5 on others, left 52 of 148 SMs idle at 12,288 atoms, and ran a small
+// box's 8 models one after the other.)
+struct Share {
+  int M, blocks, whole, left;  // whole tiles per CTA; tiles left over
+  __host__ __device__ Share(int ntiles, int M_, int blocks_)
+      : M(M_), blocks(blocks_), whole(ntiles / blocks_), left(ntiles - whole * blocks_) {}
+  // first item (of the tiles left over) of a CTA, and the CTA that has an item
+  __host__ __device__ int first(int block) const { return (int)((long long)left * M * block / blocks); }
+  __host__ __device__ int owner(int item) const {
+    const long long n = (long long)left * M;
+    return (int)(((long long)(item + 1) * blocks + n - 1) / n) - 1;
+  }
+  __host__ __device__ int most() const { return (int)(((long long)left * M + blocks - 1) / blocks); }  // items of a CTA
+};
 struct Items {
-  int M, lo, count;
+  int M, tile0, nwhole, shared0, lo, count;  // items of whole tiles; first tile left over
   __device__ void cut(int ntiles, int M_, int block, int blocks) {
+    const Share s(ntiles, M_, blocks);
     M = M_;
-    lo = first_item(ntiles, M, block, blocks);
-    count = first_item(ntiles, M, block + 1, blocks) - lo;
+    tile0 = block * s.whole;
+    nwhole = s.whole * M;
+    shared0 = s.whole * blocks;
+    lo = s.first(block);
+    count = nwhole + s.first(block + 1) - lo;
   }
   __device__ void at(int k, int& tile, int& model) const {
-    tile = (lo + k) / M;
-    model = lo + k - tile * M;
+    const int i = k < nwhole ? k : lo + k - nwhole;
+    tile = i / M;
+    model = i - tile * M;
+    tile += k < nwhole ? tile0 : shared0;
   }
 };
 
 struct Bars {
-  uint64_t x_full[kXStages], x_empty[kXStages], w_full[kWSlots], w_empty[kWSlots];
-  uint64_t acc_full[2], acc_free[2], act_ready[4], act_free, lo_free, done, ex_ready, ex_free, bias_full, bias_free;
+  uint64_t full[kChunks], empty[kChunks];
+  uint64_t acc_full[2], act_ready[4], dx_free[2], r0_free, done, bias_full, bias_free;
+  uint64_t e_fwd[8], e_back[8], e_half[4];  // row energies handed from warp to warp
   uint32_t tmem_slot;
   int abort_flag;
   Items items;
-  float ex[BM];
+  float e_row[3][2][BM];
 };
 
 // Drop the 128-byte L2 line at a (128-byte aligned) without writing it back;
@@ -244,88 +253,71 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   }
 }
 
-// Write 8 consecutive columns [n, n + 8) of row r as 16-bit hi (+ lo) into
-// the swizzled K-major activation buffer (BF16, or FP16 when F16); one paired
-// conversion per two columns for the high parts and one for the residuals.
+// 16 columns of a row as 16-bit pairs: w[0..7] the high parts, w[8..15] the
+// residuals (BF16, or FP16 when F16); one paired conversion per two columns.
 template <bool F16>
-__device__ __forceinline__ void act_store(uint8_t* act, int r, int n, const F2* v, bool with_lo) {
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float a, b;
-    unpack2(v[k], a, b);
-    if constexpr (F16) {
-      const __half2 hb = __floats2half2_rn(a, b);
-      h[k] = *reinterpret_cast<const uint32_t*>(&hb);
-    } else {
-      const __nv_bfloat162 hb = __floats2bfloat162_rn(a, b);
-      h[k] = *reinterpret_cast<const uint32_t*>(&hb);
-    }
-  }
-  uint8_t* dst = act + (n >> 6) * kAtom + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u +
-                 ((((n & 63) >> 3) ^ (r & 7)) << 4);
-  *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
-  if (!with_lo) return;
+__device__ __forceinline__ void split_pair(F2 v, bool with_lo, uint32_t& hi, uint32_t& lo) {
+  float a, b;
+  unpack2(v, a, b);
   const F2 minus = pack2(-1.f, -1.f);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float a, b;
-    if constexpr (F16) {
-      const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&h[k]));
-      unpack2(fma2(pack2(hf.x, hf.y), minus, v[k]), a, b);  // v - hi, rounded once
-      const __half2 lb = __floats2half2_rn(a, b);
-      l[k] = *reinterpret_cast<const uint32_t*>(&lb);
-    } else {
-      const float2 hf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&h[k]));
-      unpack2(fma2(pack2(hf.x, hf.y), minus, v[k]), a, b);
-      const __nv_bfloat162 lb = __floats2bfloat162_rn(a, b);
-      l[k] = *reinterpret_cast<const uint32_t*>(&lb);
-    }
+  if constexpr (F16) {
+    const __half2 hb = __floats2half2_rn(a, b);
+    hi = *reinterpret_cast<const uint32_t*>(&hb);
+    if (!with_lo) return;
+    const float2 hf = __half22float2(hb);
+    unpack2(fma2(pack2(hf.x, hf.y), minus, v), a, b);  // v - hi, rounded once
+    const __half2 lb = __floats2half2_rn(a, b);
+    lo = *reinterpret_cast<const uint32_t*>(&lb);
+  } else {
+    const __nv_bfloat162 hb = __floats2bfloat162_rn(a, b);
+    hi = *reinterpret_cast<const uint32_t*>(&hb);
+    if (!with_lo) return;
+    const float2 hf = __bfloat1622float2(hb);
+    unpack2(fma2(pack2(hf.x, hf.y), minus, v), a, b);
+    const __nv_bfloat162 lb = __floats2bfloat162_rn(a, b);
+    lo = *reinterpret_cast<const uint32_t*>(&lb);
   }
-  *reinterpret_cast<uint4*>(dst + kActHalf) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-template <bool F16>
+// Operand forms: which lo parts there are.
+enum Form { kBf16 = 0, kBf16x2 = 1, kF16 = 2 };
+template <int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedParams p) {
+  constexpr bool F16 = FORM == kF16;
+  constexpr bool a_lo = FORM != kBf16;     // forward A operands (X, H1, H2)
+  constexpr bool g_lo = FORM == kBf16x2;   // input-gradient A operands (G3, G2, G1)
+  constexpr bool wf_lo = FORM == kF16;     // forward GEMMs add A_hi x W_lo
   extern __shared__ uint8_t smem_raw[];
   // rounded up to 1024 bytes by an offset, so that accesses stay in the shared window
   uint8_t* smem = smem_raw + (0u - smem_u32(smem_raw) & 1023u);
-  uint8_t* act = smem;
-  float* xpose = reinterpret_cast<float*>(smem + kRing);
+  float* biases = reinterpret_cast<float*>(smem + kRing);
+  float* xpose = biases + 4 * kBias;
   Bars* bars = reinterpret_cast<Bars*>(smem + kSmemMain);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int M = p.n_models;
-  const int XS = p.xstages;
   const bool grad = p.ndx > 0;
-  // weight slot s: 0, 1 behind the activations, 2, 3 in the activations' lo half
-  auto slot_at = [&](int s) -> uint8_t* { return act + (s < 2 ? kActBytes + s * kWStage : kActHalf + (s - 2) * kWStage); };
-  // component at byte `off` of L1 stage s
-  auto stage_at = [&](int s, uint32_t off) -> uint8_t* {
-    uint32_t o = kXBase + s * p.xstage + off;
-    return act + (o >= kRing ? o - kRing : o);
-  };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kXStages; ++s) {
-      mbar_init(&bars->x_full[s], 1);
-      mbar_init(&bars->x_empty[s], 1);
+    for (int s = 0; s < kChunks; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1);
+    }
+    for (int s = 0; s < 8; ++s) {
+      mbar_init(&bars->e_fwd[s], 1);
+      mbar_init(&bars->e_back[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->acc_full[s], 1);
-      mbar_init(&bars->acc_free[s], kEpiWarps);
+      mbar_init(&bars->dx_free[s], kEpiWarps);
     }
-    for (int s = 0; s < kWSlots; ++s) {
-      mbar_init(&bars->w_full[s], 1);
-      mbar_init(&bars->w_empty[s], 1);
+    for (int a = 0; a < 4; ++a) {
+      mbar_init(&bars->act_ready[a], kEpiWarps);
+      mbar_init(&bars->e_half[a], 1);
     }
-    for (int a = 0; a < 4; ++a) mbar_init(&bars->act_ready[a], kEpiWarps);
-    mbar_init(&bars->act_free, 1);
-    mbar_init(&bars->lo_free, 1);
+    mbar_init(&bars->r0_free, kEpiWarps);
     mbar_init(&bars->done, 1);
-    mbar_init(&bars->ex_ready, BM);
-    mbar_init(&bars->ex_free, BM);
     mbar_init(&bars->bias_full, 1);
     mbar_init(&bars->bias_free, kEpiWarps);
     bars->abort_flag = 0;
@@ -343,291 +335,319 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
   // wave; every role reads or writes global memory only after this wait.
   pdl_wait();
 
-  // L1 stage layout: A hi | A lo | B hi | B lo, each `unit` columns wide
-  const uint32_t xa = BM * p.unit * 2, xb = (uint32_t)p.d1 * p.unit * 2, xb_slot = 256u * p.unit * 2;
-  const uint32_t x_tx = xa * (1 + p.a_lo) + xb * (1 + p.wf_lo);
+  // The producer and the MMA issuer run warp-wide, one elected lane issuing the
+  // copies, MMAs and commits: their operands are then warp-uniform, where a
+  // single thread's would be moved to uniform registers one by one.  (With one
+  // thread and a table of ring places in shared memory the issue itself was the
+  // bound: 1.2k cycles for the four copies of an L1 chunk, 620 for the four MMAs
+  // of a B1 chunk.)
+  auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, p.err, p.timeout_ns));
+  };
+  // Ring places: components one after the other, none across the end.  The
+  // producer and the issuer work them out alike.
+  auto place = [](uint32_t& pos, uint32_t bytes) -> uint32_t {
+    const uint32_t at = pos + bytes > kRing ? 0 : pos;
+    pos = at + bytes;
+    return at;
+  };
+  const uint32_t xa = BM * kUnit * 2, xb = (uint32_t)p.d1 * kUnit * 2;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
+    // Every chunk in the order the GEMMs take them, as far ahead as the ring
+    // holds: the next item's L1 streams in while this one's gradient runs.
     // (with p.stall it issues nothing: the other roles' waits run out)
-    if (lane == 0 && !p.stall) {
+    if (!p.stall) {
+      const bool leader = elect_one();
       const uint64_t keep = l2_evict_last();
-      uint32_t x_used = 0, x_par = 0;  // per L1 stage: used before; parity of its next use
-      uint32_t w_used = 0, w_par = 0;  // the same per weight slot
-      int bias_loaded = 0;
+      uint32_t seq = 0, oldest = 0;  // next chunk, oldest chunk not known to be consumed
+      uint32_t pos = 0;
+      int room = kRing, taken = 0, size = 0;  // bytes free; of this chunk; of the chunk in slot `lane`
+      int biases_loaded = 0;
       bool ok = true;
-      // the latest copy into slot s has been multiplied
-      auto slot_free = [&](int s) -> bool {
-        return !((w_used >> s) & 1) ||
-               wait_bar(&bars->w_empty[s], ((w_par >> s) & 1) ^ 1, abort_flag, p.err, p.timeout_ns);
-      };
-      auto stage_free = [&](int s) -> bool {
-        return !((x_used >> s) & 1) ||
-               wait_bar(&bars->x_empty[s], ((x_par >> s) & 1) ^ 1, abort_flag, p.err, p.timeout_ns);
-      };
-      auto take_slot = [&](int s, uint32_t bytes) -> bool {
-        if (!slot_free(s)) return false;
-        w_used |= 1u << s;
-        w_par ^= 1u << s;
-        mbar_expect_tx(&bars->w_full[s], bytes);
+      auto retire = [&]() -> bool {
+        const uint32_t s = oldest % kChunks;
+        if (!wait_all(&bars->empty[s], (oldest / kChunks) & 1)) return false;
+        room += __shfl_sync(0xffffffffu, size, s);
+        ++oldest;
         return true;
+      };
+      // starts a chunk of `bytes` in all: its barrier, and what it takes of the ring
+      auto open = [&](uint32_t bytes) -> bool {
+        while (seq - oldest >= kChunks)
+          if (!retire()) return false;
+        if (leader) mbar_expect_tx(&bars->full[seq % kChunks], bytes);
+        taken = 0;
+        return true;
+      };
+      // place of a component, once it is free
+      auto room_for = [&](uint32_t bytes, uint32_t& at) -> bool {
+        const uint32_t before = pos;
+        at = place(pos, bytes);
+        const int used = (int)bytes + (at == 0 && before != 0 ? (int)(kRing - before) : 0);
+        room -= used;
+        taken += used;
+        while (room < 0)
+          if (!retire()) return false;
+        return true;
+      };
+      auto load = [&](const CUtensorMap* map, int x, int y, uint32_t bytes) -> bool {
+        uint32_t at;
+        if (!room_for(bytes, at)) return false;
+        if (leader) tma_load_2d(map, &bars->full[seq % kChunks], smem + at, x, y);
+        return true;
+      };
+      // the AEV tile is read once per model: kept in L2 ahead of other lines
+      auto load_keep = [&](const CUtensorMap* map, int x, int y, uint32_t bytes) -> bool {
+        uint32_t at;
+        if (!room_for(bytes, at)) return false;
+        if (leader) tma_load_2d_hint(map, &bars->full[seq % kChunks], smem + at, x, y, keep);
+        return true;
+      };
+      auto close = [&]() {
+        if (lane == (int)(seq % kChunks)) size = taken;
+        ++seq;
       };
       for (int it = 0; it < items.count && ok; ++it) {
         int tile, m;
         items.at(it, tile, m);
         const int row0 = p.tile_row[tile];
         const int g = m * p.n_species + p.tile_species[tile];
-        bool act_ok = it == 0;  // the previous item's last GEMM has read the activations
-        for (int u = 0; u < p.nunits; ++u) {
-          const int s = u % XS;
-          if (u < XS) {
-            // first use in this item: what the previous item kept there must have been read
-            if (!act_ok && (p.stage_slots[s] & 16u)) {
-              if (!(ok = wait_bar(&bars->act_free, (it - 1) & 1, abort_flag, p.err, p.timeout_ns))) break;
-              act_ok = true;
-            }
-            if (!act_ok)
-              for (int q = 0; q < kWSlots && ok; ++q)
-                if ((p.stage_slots[s] >> q) & 1) ok = slot_free(q);
-            if (!ok) break;
-          }
-          if (!(ok = stage_free(s))) break;
-          x_used |= 1u << s;
-          x_par ^= 1u << s;
-          const int c = p.xunit[u] * p.unit;
-          mbar_expect_tx(&bars->x_full[s], x_tx);
-          // the AEV tile is read once per model: kept in L2 ahead of other lines
-          tma_load_2d_hint(&maps.x, &bars->x_full[s], stage_at(s, 0), c, row0, keep);
-          if (p.a_lo) tma_load_2d_hint(&maps.xlo, &bars->x_full[s], stage_at(s, xa), c, row0, keep);
-          tma_load_2d(&maps.w1t, &bars->x_full[s], stage_at(s, 2 * xa), c, g * p.d1);
-          if (p.wf_lo) tma_load_2d(&maps.w1t_lo, &bars->x_full[s], stage_at(s, 2 * xa + xb_slot), c, g * p.d1);
+        for (int u = 0; u < p.nunits && ok; ++u) {
+          const int c = p.xunit[u] * kUnit;
+          ok = open(xa * (1 + a_lo) + xb * (1 + wf_lo)) && load_keep(&maps.x, c, row0, xa) &&
+               (!a_lo || load_keep(&maps.xlo, c, row0, xa)) && load(&maps.w1t, c, g * p.d1, xb) &&
+               (!wf_lo || load(&maps.w1t_lo, c, g * p.d1, xb));
+          if (ok) close();
         }
         if (!ok) break;
         // the item's biases and last kernel
-        if (it > 0 && !(ok = wait_bar(&bars->bias_free, (it - 1) & 1, abort_flag, p.err, p.timeout_ns))) break;
-        mbar_expect_tx(&bars->bias_full, (uint32_t)(p.d1 + p.d2 + 2 * p.d3) * 4);
-        bulk_load(&bars->bias_full, xpose, p.b1 + (size_t)g * p.d1, p.d1 * 4);
-        bulk_load(&bars->bias_full, xpose + kBias, p.b2 + (size_t)g * p.d2, p.d2 * 4);
-        bulk_load(&bars->bias_full, xpose + 2 * kBias, p.b3 + (size_t)g * p.d3, p.d3 * 4);
-        bulk_load(&bars->bias_full, xpose + 3 * kBias, p.w4 + (size_t)g * p.d3, p.d3 * 4);
-        bias_loaded = it + 1;
-        // weight chunks of the remaining GEMMs, in MMA order
-        // (a GEMM with weight low parts takes the hi and lo chunks of each K step)
-        const CUtensorMap* wm[4] = {&maps.w2t, &maps.w3t, &maps.w3, &maps.w2};
-        const CUtensorMap* wml[4] = {&maps.w2t_lo, &maps.w3t_lo, &maps.w3_lo, &maps.w2_lo};
-        const int rows_g[4] = {p.d2, p.d3, p.d2, p.d1};
-        const int nk[4] = {p.d1 / BK, p.d2 / BK, p.d3 / BK, p.d2 / BK};
-        int q = 0;
-        bool lo_ok = false;  // L3 has read the activations' lo half
-        // slots 2 and 3 may be filled once L3 has run
-        auto back_slot = [&](uint32_t bytes) -> int {
-          const int s = q++ & (p.bslots - 1);
-          if (s >= 2 && !lo_ok) {
-            if (!wait_bar(&bars->lo_free, it & 1, abort_flag, p.err, p.timeout_ns)) return -1;
-            lo_ok = true;
-          }
-          return take_slot(s, bytes) ? s : -1;
-        };
-        for (int jb = 0; jb < (grad ? 4 : 2) && ok; ++jb) {
-          if (jb == 2) q = 0;
-          for (int kc = 0; kc < nk[jb] && ok; ++kc) {
-            for (int t = 0; t < 1 + (jb < 2 ? p.wf_lo : p.wb_lo); ++t) {
-              const uint32_t bytes = (uint32_t)rows_g[jb] * BK * 2;
-              int s;
-              if (jb < 2) {
-                s = q & 1;
-                if (q < 2)  // the L1 stages that overlap the slot have been read
-                  for (int xs = 0; xs < XS && ok; ++xs)
-                    if ((p.slot_stages[s] >> xs) & 1) ok = stage_free(xs);
-                ++q;
-                if (!ok || !(ok = take_slot(s, bytes))) break;
-              } else {
-                s = back_slot(bytes);
-                if (!(ok = s >= 0)) break;
-              }
-              tma_load_2d(t ? wml[jb] : wm[jb], &bars->w_full[s], slot_at(s), kc * BK, g * rows_g[jb]);
-            }
-          }
+        if (it > 0 && !(ok = wait_all(&bars->bias_free, (it - 1) & 1))) break;
+        if (leader) {
+          mbar_expect_tx(&bars->bias_full, (uint32_t)(p.d1 + p.d2 + 2 * p.d3) * 4);
+          bulk_load(&bars->bias_full, biases, p.b1 + (size_t)g * p.d1, p.d1 * 4);
+          bulk_load(&bars->bias_full, biases + kBias, p.b2 + (size_t)g * p.d2, p.d2 * 4);
+          bulk_load(&bars->bias_full, biases + 2 * kBias, p.b3 + (size_t)g * p.d3, p.d3 * 4);
+          bulk_load(&bars->bias_full, biases + 3 * kBias, p.w4 + (size_t)g * p.d3, p.d3 * 4);
         }
-        // B1: the W1 rows of up to 16 dX column groups per run, stacked in the
-        // slot; four groups of an aligned 64-column chunk take one box
-        for (int r0 = 0; r0 < p.ndx && ok; r0 += 16) {
-          const int ng = min(16, p.ndx - r0);
-          for (int kc = 0; kc < p.d1 / BK && ok; ++kc) {
-            for (int t = 0; t < 1 + p.wb_lo; ++t) {
-              const int s = back_slot((uint32_t)ng * kGroup * BK * 2);
-              if (!(ok = s >= 0)) break;
-              for (int i = 0; i < ng;) {
-                const int gr = p.dgroup[r0 + i];
-                const bool four = (gr & 3) == 0 && i + 4 <= ng && p.dgroup[r0 + i + 3] == gr + 3;
-                const CUtensorMap* mp = four ? (t ? &maps.w1_lo : &maps.w1) : (t ? &maps.w1g_lo : &maps.w1g);
-                tma_load_2d(mp, &bars->w_full[s], slot_at(s) + i * kGroup * BK * 2, kc * BK, g * p.d0 + gr * kGroup);
-                i += four ? 4 : 1;
+        biases_loaded = it + 1;
+        // weight chunks of the remaining GEMMs, in MMA order: a K step of 64 each
+        auto weights = [&](const CUtensorMap* hi, const CUtensorMap* lo, int rows, int k, bool with_lo) -> bool {
+          const uint32_t bytes = (uint32_t)rows * BK * 2;
+          for (int kc = 0; kc < k; kc += BK) {
+            if (!open(bytes * (1 + with_lo)) || !load(hi, kc, g * rows, bytes) ||
+                (with_lo && !load(lo, kc, g * rows, bytes)))
+              return false;
+            close();
+          }
+          return true;
+        };
+        ok = weights(&maps.w2t, &maps.w2t_lo, p.d2, p.d1, wf_lo) && weights(&maps.w3t, &maps.w3t_lo, p.d3, p.d2, wf_lo);
+        if (!ok) break;
+        if (!grad) continue;
+        ok = weights(&maps.w3, &maps.w3_lo, p.d2, p.d3, p.wb_lo) && weights(&maps.w2, &maps.w2_lo, p.d1, p.d2, p.wb_lo);
+        // B1: the W1 rows of the run's dX column groups, stacked: boxes of 4, 2
+        // or 1 neighbouring groups
+        int b0 = 0;
+        for (int r0 = 0; r0 < p.ndx && ok; r0 += kRunGroups) {
+          const uint32_t bytes = (uint32_t)min(kRunGroups, p.ndx - r0) * kGroup * BK * 2;
+          int b = b0;
+          for (int kc = 0; kc < p.d1 && ok; kc += BK) {
+            ok = open(bytes * (1 + p.wb_lo));
+            for (int t = 0; t < 1 + p.wb_lo && ok; ++t) {
+              uint32_t at;
+              if (!(ok = room_for(bytes, at))) break;
+              b = b0;
+              for (uint32_t off = 0; off < bytes; ++b) {
+                const uint32_t n = p.box_n[b];
+                const CUtensorMap* mp = n == 4 ? (t ? &maps.w1_lo : &maps.w1)
+                                               : (n == 2 ? (t ? &maps.w1p_lo : &maps.w1p) : (t ? &maps.w1g_lo : &maps.w1g));
+                if (leader)
+                  tma_load_2d(mp, &bars->full[seq % kChunks], smem + at + off, kc, g * p.d0 + p.box_g[b] * kGroup);
+                off += n * kGroup * BK * 2;
               }
             }
+            if (ok) close();
           }
+          b0 = b;
         }
       }
       // Before the CTA can exit, every issued TMA load must have landed (on an
-      // abort some stages may never be consumed).  Bounded, ignores the abort flag.
-      int dummy = 0;
-      for (int s = 0; s < XS; ++s)
-        if ((x_used >> s) & 1) wait_bar(&bars->x_full[s], ((x_par >> s) & 1) ^ 1, &dummy, p.err, p.timeout_ns);
-      for (int s = 0; s < kWSlots; ++s)
-        if ((w_used >> s) & 1) wait_bar(&bars->w_full[s], ((w_par >> s) & 1) ^ 1, &dummy, p.err, p.timeout_ns);
-      if (bias_loaded) wait_bar(&bars->bias_full, (bias_loaded - 1) & 1, &dummy, p.err, p.timeout_ns);
+      // abort some chunks may never be consumed, the last one not be complete).
+      // Bounded, ignores the abort flag.
+      if (leader) {
+        int dummy = 0;
+        const uint32_t end = seq + (ok ? 0 : 1);
+        for (uint32_t k = end > kChunks ? end - kChunks : 0; k < end; ++k)
+          wait_bar(&bars->full[k % kChunks], (k / kChunks) & 1, &dummy, p.err, p.timeout_ns);
+        if (biases_loaded) wait_bar(&bars->bias_full, (biases_loaded - 1) & 1, &dummy, p.err, p.timeout_ns);
+      }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      uint32_t x_par = 0, w_par = 0, act_par = 0;  // parities of the next full phase (bit per stage, slot, atom)
-      uint32_t job = 0;
-      bool ok = true;
-      const uint32_t act_hi = smem_u32(act), act_lo = smem_u32(act + kActHalf);
-      auto acquire_acc = [&](uint32_t b) -> bool {
-        return job < 2 || wait_bar(&bars->acc_free[b], ((job >> 1) - 1) & 1, abort_flag, p.err, p.timeout_ns);
-      };
-      auto wait_slot = [&](int s) -> bool {
-        if (!wait_bar(&bars->w_full[s], (w_par >> s) & 1, abort_flag, p.err, p.timeout_ns)) return false;
-        w_par ^= 1u << s;
-        fence_after_sync();
-        return true;
-      };
-      int q = 0;  // weight chunks taken since the slots were restarted
-      // one GEMM whose A operand is the activation buffer (K/64 atoms) and B the
-      // weight slots.  With wait_act, each K-atom is used as soon as the epilogue
-      // has published it, so the GEMM overlaps the epilogue that feeds it.
-      // alo: A carries a lo part; wlo: each K step also has a W lo chunk.
-      auto gemm_act = [&](int n, int k, uint32_t b, int slots, bool wait_act, bool alo, bool wlo) -> bool {
-        const uint32_t idesc = F16 ? idesc_f16_f32(n) : idesc_bf16_f32(n);
-        const uint32_t d = tmem + b * 256;
-        for (int kc = 0; kc < k / BK; ++kc) {
-          if (wait_act) {
-            if (!wait_bar(&bars->act_ready[kc], (act_par >> kc) & 1, abort_flag, p.err, p.timeout_ns)) return false;
-            act_par ^= 1u << kc;
-          }
-          int s = q++ & (slots - 1);
-          if (!wait_slot(s)) return false;
-          uint32_t bs = smem_u32(slot_at(s));
+    // Tensor memory: two regions of 256 columns.  L1 -> R0, L2 -> R1, L3 -> R0,
+    // B3 -> R1, B2 -> R0, B1 runs -> the halves of R1 in turn; the A operand of
+    // each GEMM but L1 is the other region, where the epilogue has put it over
+    // the accumulator it came from.  So a region is overwritten only by a GEMM
+    // whose own A operand was made from the result of the last reader; what that
+    // leaves open (the next item's L1 and L2, B1 halves) is waited for.
+    const bool leader = elect_one();
+    uint32_t seq = 0, pos = 0;      // next chunk and its place in the ring
+    uint32_t act_par = 0;           // parity of the atoms' next phases
+    uint32_t job = 0, runs = 0;     // accumulators committed; B1 runs issued
+    bool ok = true;
+    auto take = [&]() -> bool {
+      if (!wait_all(&bars->full[seq % kChunks], (seq / kChunks) & 1)) return false;
+      fence_after_sync();
+      return true;
+    };
+    auto give = [&]() {
+      if (leader) mma_commit(&bars->empty[seq % kChunks]);
+      ++seq;
+    };
+    auto finish = [&]() {
+      if (leader) mma_commit(&bars->acc_full[job & 1]);
+      ++job;
+    };
+    // shared-memory descriptors: constant high word, start address in the low one
+    const uint32_t base = smem_u32(smem);
+    auto desc = [&](uint32_t at, uint32_t hi) -> uint64_t { return sdesc_of((base + at) >> 4, hi); };
+    const uint32_t hi128 = sdesc_hi128(), hi64 = sdesc_hi64();
+    // D (n columns at d) = A (k columns, in tensor memory at a) x the weight chunks.
+    // With wait_act, each K-atom is used as soon as the epilogue has published
+    // it, so the GEMM overlaps the epilogue that feeds it.
+    // alo: A carries a lo part; wlo: each chunk also has the W lo part.
+    auto gemm_act = [&](int n, int k, uint32_t d, uint32_t a, bool wait_act, bool alo, bool wlo) -> bool {
+      const uint32_t idesc = F16 ? idesc_f16_f32(n) : idesc_bf16_f32(n);
+      const uint32_t bytes = (uint32_t)n * BK * 2;
+      for (int kc = 0; kc < k / BK; ++kc) {
+        if (wait_act) {
+          if (!wait_all(&bars->act_ready[kc], (act_par >> kc) & 1)) return false;
+          act_par ^= 1u << kc;
+        }
+        if (!take()) return false;
+        const uint64_t bh = desc(place(pos, bytes), hi128);
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t bd = sdesc_sw128(bs + kk * 32);
-            mma_bf16(d, sdesc_sw128(act_hi + kc * kAtom + kk * 32), bd, idesc, (kc | kk) != 0);
-            if (alo) mma_bf16(d, sdesc_sw128(act_lo + kc * kAtom + kk * 32), bd, idesc, 1u);
+            mma_ts(d, a + 64 * kc + 16 * kk, bh + 2 * kk, idesc, (kc | kk) != 0);
+            if (alo) mma_ts(d, a + 64 * kc + 16 * kk + 8, bh + 2 * kk, idesc, 1u);
           }
-          mma_commit(&bars->w_empty[s]);
-          if (wlo) {
-            s = q++ & (slots - 1);
-            if (!wait_slot(s)) return false;
-            bs = smem_u32(slot_at(s));
+        }
+        if (wlo) {
+          const uint64_t bl = desc(place(pos, bytes), hi128);
+          if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk)
-              mma_bf16(d, sdesc_sw128(act_hi + kc * kAtom + kk * 32), sdesc_sw128(bs + kk * 32), idesc, 1u);
-            mma_commit(&bars->w_empty[s]);
+            for (int kk = 0; kk < BK / 16; ++kk) mma_ts(d, a + 64 * kc + 16 * kk, bl + 2 * kk, idesc, 1u);
           }
         }
-        return true;
-      };
-      for (int it = 0; it < items.count && ok; ++it) {
-        // L1: A and B from the X ring; K steps of columns that are zero in every row are left out
-        {
-          const uint32_t b = job & 1;
-          if (!(ok = acquire_acc(b))) break;
-          const uint32_t idesc = F16 ? idesc_f16_f32(p.d1) : idesc_bf16_f32(p.d1);
-          const uint32_t d = tmem + b * 256;
-          uint32_t started = 0;
-          for (int u = 0; u < p.nunits; ++u) {
-            const int s = u % XS;
-            if (!(ok = wait_bar(&bars->x_full[s], (x_par >> s) & 1, abort_flag, p.err, p.timeout_ns))) break;
-            x_par ^= 1u << s;
-            fence_after_sync();
-            const uint32_t ah = smem_u32(stage_at(s, 0)), al = smem_u32(stage_at(s, xa));
-            const uint32_t bh = smem_u32(stage_at(s, 2 * xa)), bl = smem_u32(stage_at(s, 2 * xa + xb_slot));
-            const uint32_t bits = p.xbits[u];
-            for (int kk = 0; kk < p.unit / 16; ++kk) {
-              if (!((bits >> kk) & 1)) continue;
-              const uint64_t ad = p.unit == 64 ? sdesc_sw128(ah + kk * 32) : sdesc_sw64(ah + kk * 32);
-              const uint64_t bd = p.unit == 64 ? sdesc_sw128(bh + kk * 32) : sdesc_sw64(bh + kk * 32);
-              mma_bf16(d, ad, bd, idesc, started);
-              started = 1;
-              if (p.a_lo) mma_bf16(d, p.unit == 64 ? sdesc_sw128(al + kk * 32) : sdesc_sw64(al + kk * 32), bd, idesc, 1u);
-              if (p.wf_lo) mma_bf16(d, ad, p.unit == 64 ? sdesc_sw128(bl + kk * 32) : sdesc_sw64(bl + kk * 32), idesc, 1u);
-            }
-            mma_commit(&bars->x_empty[s]);
-          }
-          if (!ok) break;
-          mma_commit(&bars->acc_full[b]);
-          ++job;
-        }
-        // L2, L3, B3, B2: A from the activation buffer written by the epilogue
-        const int ns[4] = {p.d2, p.d3, p.d2, p.d1};
-        const int ks[4] = {p.d1, p.d2, p.d3, p.d2};
-        q = 0;
-        for (int jb = 0; jb < (grad ? 4 : 2) && ok; ++jb) {
-          const uint32_t b = job & 1;
-          const bool fwd = jb < 2;
-          if (jb == 2) q = 0;
-          if (!(ok = acquire_acc(b))) break;
-          if (!(ok = gemm_act(ns[jb], ks[jb], b, fwd ? 2 : p.bslots, true, fwd ? p.a_lo : p.g_lo,
-                              fwd ? p.wf_lo : p.wb_lo)))
-            break;
-          mma_commit(&bars->acc_full[b]);
-          if (jb == 1 && grad) mma_commit(&bars->lo_free);
-          ++job;
-        }
-        if (!ok) break;
-        // B1: dX on runs of up to 16 column groups (<= 256 columns), A = G1
-        // (published atom by atom for the first run)
-        for (int r0 = 0; r0 < p.ndx && ok; r0 += 16) {
-          const uint32_t b = job & 1;
-          if (!(ok = acquire_acc(b))) break;
-          if (!(ok = gemm_act(kGroup * min(16, p.ndx - r0), p.d1, b, p.bslots, r0 == 0, p.g_lo, p.wb_lo))) break;
-          mma_commit(&bars->acc_full[b]);
-          ++job;
-        }
-        if (!ok) break;
-        mma_commit(&bars->act_free);
+        give();
       }
-      // all issued MMAs complete before TMEM is released
-      mma_commit(&bars->done);
-      wait_bar(&bars->done, 0, abort_flag, p.err, p.timeout_ns);
+      return true;
+    };
+    // the halves of R1 that hold dX have been read
+    auto dx_read = [&](uint32_t half) -> bool {
+      const uint32_t uses = (runs + 1 - half) >> 1;
+      return uses == 0 || wait_all(&bars->dx_free[half], (uses - 1) & 1);
+    };
+    const uint32_t R0 = tmem, R1 = tmem + 256;
+    for (int it = 0; it < items.count && ok; ++it) {
+      // L1: A and B from the ring; K steps of columns that are zero in every row are left out
+      if (it > 0) {
+        // B1 has read R0 (energies only: the epilogue has)
+        ok = grad ? wait_all(&bars->acc_full[(job - 1) & 1], ((job - 1) >> 1) & 1) : wait_all(&bars->r0_free, (it - 1) & 1);
+        if (!ok) break;
+        fence_after_sync();
+      }
+      {
+        const uint32_t idesc = F16 ? idesc_f16_f32(p.d1) : idesc_bf16_f32(p.d1);
+        uint32_t started = 0;
+        for (int u = 0; u < p.nunits; ++u) {
+          if (!(ok = take())) break;
+          const uint64_t ah = desc(place(pos, xa), hi64), al = a_lo ? desc(place(pos, xa), hi64) : 0ull;
+          const uint64_t bh = desc(place(pos, xb), hi64), bl = wf_lo ? desc(place(pos, xb), hi64) : 0ull;
+          const uint32_t bits = p.xbits[u];
+#pragma unroll
+          for (int kk = 0; kk < kUnit / 16; ++kk) {
+            if (!((bits >> kk) & 1)) continue;
+            if (leader) {
+              mma_bf16(R0, ah + 2 * kk, bh + 2 * kk, idesc, started);
+              if (a_lo) mma_bf16(R0, al + 2 * kk, bh + 2 * kk, idesc, 1u);
+              if (wf_lo) mma_bf16(R0, ah + 2 * kk, bl + 2 * kk, idesc, 1u);
+            }
+            started = 1;
+          }
+          give();
+        }
+        if (!ok) break;
+        finish();
+      }
+      // L2, L3, B3, B2
+      if (!(ok = dx_read(0) && dx_read(1))) break;
+      fence_after_sync();
+      ok = gemm_act(p.d2, p.d1, R1, R0, true, a_lo, wf_lo);
+      if (!ok) break;
+      finish();
+      ok = gemm_act(p.d3, p.d2, R0, R1, true, a_lo, wf_lo);
+      if (!ok) break;
+      finish();
+      if (!grad) continue;
+      ok = gemm_act(p.d2, p.d3, R1, R0, true, g_lo, p.wb_lo);
+      if (!ok) break;
+      finish();
+      ok = gemm_act(p.d1, p.d2, R0, R1, true, g_lo, p.wb_lo);
+      if (!ok) break;
+      finish();
+      // B1: dX on runs of up to 8 column groups (<= 128 columns), A = G1
+      // (published atom by atom for the first run)
+      for (int r0 = 0; r0 < p.ndx && ok; r0 += kRunGroups) {
+        const uint32_t half = runs & 1;
+        if (!(ok = dx_read(half))) break;
+        fence_after_sync();
+        if (!(ok = gemm_act(kGroup * min(kRunGroups, p.ndx - r0), p.d1, R1 + 128 * half, R0, r0 == 0, g_lo, p.wb_lo))) break;
+        finish();
+        ++runs;
+      }
     }
+    // all issued MMAs complete before TMEM is released
+    if (leader) mma_commit(&bars->done);
+    wait_bar(&bars->done, 0, abort_flag, p.err, p.timeout_ns);
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue
     // Warp (q, part) owns rows [32 q, 32 q + 32) and, of every 64-column
-    // K-atom, the columns [16 part, 16 part + 16): the 16 warps finish the
-    // atoms one after the other, and the next GEMM starts on the first.
+    // K-atom, the columns [16 part, 16 part + 16) (one MMA K step): it turns
+    // the accumulator's 16 columns into the 8 + 8 columns of packed 16-bit hi
+    // and lo parts that the next GEMM reads as its A operand, in place.  The
+    // 16 warps finish the atoms one after the other, and the next GEMM starts
+    // on the first.
     const int q = warp & 3;
     const int part = (warp - 2) >> 2;
     const int r = 32 * q + lane;
-    const uint32_t lane_base = (uint32_t)(32 * q) << 16;
-    uint32_t job = 0;  // accumulators taken; they alternate between the two buffers
+    const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
+    uint32_t job = 0, runs = 0;
     bool ok = true;
     // per-CTA CELU' scratch [(d1 + d2) / 4][128 rows][4]: 16 bytes of a thread, 512 of a warp
     float4* dc = reinterpret_cast<float4*>(p.dc + (size_t)blockIdx.x * BM * (p.d1 + p.d2)) + r;
-    float4* xs = reinterpret_cast<float4*>(p.xs + (size_t)blockIdx.x * 2 * BM * p.d0) + r;  // the dX sums, laid out alike
-    const float* dc_lines = p.dc + (size_t)blockIdx.x * BM * (p.d1 + p.d2) + 128 * q;
     const float k2 = 1.4426950408889634f / p.alpha;  // log2(e) / alpha
     const F2 k2p = pack2(k2, k2), alp = pack2(p.alpha, p.alpha), nalp = pack2(-p.alpha, -p.alpha);
-    const bool with_lo = p.a_lo != 0;    // forward activations
-    const bool grad_lo = p.g_lo != 0;    // input-gradient operands
-    auto take_acc = [&](uint32_t b) -> bool {
-      bool ready = __all_sync(0xffffffffu, wait_bar(&bars->acc_full[b], (job >> 1) & 1, abort_flag, p.err, p.timeout_ns));
+    auto take_acc = [&]() -> bool {
+      const bool ready = wait_all(&bars->acc_full[job & 1], (job >> 1) & 1);
+      ++job;
       if (ready) fence_after_sync();
       return ready;
     };
-    auto release_acc = [&](uint32_t b) {
-      fence_before_sync();
+    auto arrive = [&](uint64_t* bar) {
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_free[b]);
-      ++job;
+      if (lane == 0) mbar_arrive(bar);
     };
-    // the 16 columns of K-atom a written by this warp are visible to the MMA
-    // (async proxy); the atom is complete when all epilogue warps arrived
+    // this warp's 16 columns of K-atom a are in tensor memory
     auto publish_atom = [&](int a) {
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->act_ready[a]);
+      tmem_wait_st();
+      fence_before_sync();
+      arrive(&bars->act_ready[a]);
     };
     // four FP32 values (two pairs) of a uniform shared address
     auto load4 = [&](const float* a, F2& lo, F2& hi) {
@@ -635,50 +655,49 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
       lo = pack2(t.x, t.y);
       hi = pack2(t.z, t.w);
     };
-    // H = celu(Z / s_W + bias) -> act for columns [0, n); celu'(z) / s_W' -> dc
-    // columns [dc0, dc0 + n), where s_W' is the scale of the weights the
-    // input gradient of this layer is taken through (a power of two, so the
-    // product is exact).  inv_s = 1 / s_W, dscale = 1 / s_W' (1 for the BF16
-    // forms).
-    auto celu_layer = [&](const float* bias /* shared */, int n, int dc0, float inv_s, float dscale) -> bool {
-      const uint32_t b = job & 1;
+    // H = celu(Z / s_W + bias) over columns [0, n) of the accumulator at `at`;
+    // celu'(z) / s_W' -> dc columns [dc0, dc0 + n), where s_W' is the scale of
+    // the weights the input gradient of this layer is taken through (a power of
+    // two, so the product is exact).  inv_s = 1 / s_W, dscale = 1 / s_W' (1 for
+    // the BF16 forms).
+    auto celu_layer = [&](uint32_t at, const float* bias /* shared */, int n, int dc0, float inv_s, float dscale) -> bool {
       const F2 isp = pack2(inv_s, inv_s), dsp = pack2(dscale, dscale);
-      if (!take_acc(b)) return false;
+      if (!take_acc()) return false;
 #pragma unroll 1
       for (int a = 0; a < n / 64; ++a) {
         const int c = 64 * a + 16 * part;
         float v[16];
-        tmem_ld16(tmem + b * 256 + lane_base + c, v);
+        tmem_ld16(at + c, v);
+        uint32_t w[16];
         float4* dst = dc + (size_t)((dc0 + c) / 4) * BM;
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          F2 bb[4], h[4], dh[4];
-          load4(bias + c + 8 * hf, bb[0], bb[1]);
-          load4(bias + c + 8 * hf + 4, bb[2], bb[3]);
+        for (int k = 0; k < 4; ++k) {
+          F2 bb[2], h[2], dh[2];
+          load4(bias + c + 4 * k, bb[0], bb[1]);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            celu_pair2(fma2(pack2(v[8 * hf + 2 * k], v[8 * hf + 2 * k + 1]), isp, bb[k]), alp, nalp, k2p, h[k], dh[k]);
-          act_store<F16>(act, r, c + 8 * hf, h, with_lo);
+          for (int u = 0; u < 2; ++u) {
+            celu_pair2(fma2(pack2(v[4 * k + 2 * u], v[4 * k + 2 * u + 1]), isp, bb[u]), alp, nalp, k2p, h[u], dh[u]);
+            split_pair<F16>(h[u], a_lo, w[2 * k + u], w[8 + 2 * k + u]);
+          }
           if (grad) {
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              float4 t;
-              unpack2(mul2(dh[2 * k], dsp), t.x, t.y);
-              unpack2(mul2(dh[2 * k + 1], dsp), t.z, t.w);
-              dst[(2 * hf + k) * BM] = t;
-            }
+            float4 t;
+            unpack2(mul2(dh[0], dsp), t.x, t.y);
+            unpack2(mul2(dh[1], dsp), t.z, t.w);
+            dst[k * BM] = t;
           }
         }
+        if constexpr (a_lo)
+          tmem_st16(at + c, w);
+        else
+          tmem_st8(at + c, w);
         publish_atom(a);
       }
-      release_acc(b);
       return true;
     };
-    // G = D / s_W * celu'(z) -> act for columns [0, n), celu'(z) / s_W read
-    // back from dc columns [dc0, dc0 + n) (written by this thread) an atom
-    // ahead, the first before the accumulator is waited for.
-    auto mask_layer = [&](int n, int dc0) -> bool {
-      const uint32_t b = job & 1;
+    // G = D / s_W * celu'(z) over columns [0, n) of the accumulator at `at`,
+    // celu'(z) / s_W read back from dc columns [dc0, dc0 + n) (written by this
+    // thread) an atom ahead, the first before the accumulator is waited for.
+    auto mask_layer = [&](uint32_t at, int n, int dc0) -> bool {
       const int na = n / 64;
       const float4* src = dc + (size_t)((dc0 + 16 * part) / 4) * BM;
       float4 dd[4];
@@ -687,43 +706,47 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
         for (int k = 0; k < 4; ++k) dd[k] = src[(16 * a + k) * BM];
       };
       fetch(0);
-      if (!take_acc(b)) return false;
+      if (!take_acc()) return false;
 #pragma unroll 1
       for (int a = 0; a < na; ++a) {
         const int c = 64 * a + 16 * part;
         float v[16];
-        tmem_ld16(tmem + b * 256 + lane_base + c, v);
-        F2 gg[8];
+        tmem_ld16(at + c, v);
+        uint32_t w[16];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          gg[2 * k] = mul2(pack2(v[4 * k], v[4 * k + 1]), pack2(dd[k].x, dd[k].y));
-          gg[2 * k + 1] = mul2(pack2(v[4 * k + 2], v[4 * k + 3]), pack2(dd[k].z, dd[k].w));
+          split_pair<F16>(mul2(pack2(v[4 * k], v[4 * k + 1]), pack2(dd[k].x, dd[k].y)), g_lo, w[2 * k], w[8 + 2 * k]);
+          split_pair<F16>(mul2(pack2(v[4 * k + 2], v[4 * k + 3]), pack2(dd[k].z, dd[k].w)), g_lo, w[2 * k + 1],
+                          w[9 + 2 * k]);
         }
         if (a + 1 < na) fetch(a + 1);
-        act_store<F16>(act, r, c, gg, grad_lo);
-        act_store<F16>(act, r, c + 8, gg + 4, grad_lo);
+        if constexpr (g_lo)
+          tmem_st16(at + c, w);
+        else
+          tmem_st8(at + c, w);
         publish_atom(a);
         // the warp has read these 16 columns of its 32 rows for the last time
         // (16 lines): they are dropped from L2 without a write-back (the next
         // item rewrites them before reading)
         if (lane < 16)
-          discard_l2(dc_lines + (size_t)((dc0 + c) / 4 + (lane >> 2)) * BM * 4 + 32 * (lane & 3));
+          discard_l2(dc - lane + ((dc0 + c) / 4 + (lane >> 2)) * BM + 8 * (lane & 3));
       }
-      release_acc(b);
       return true;
     };
+    // Row energies: a row's terms are summed in the order of 32-column chunks
+    // 0, 2, .. and 1, 3, .. of its atoms (two sums), each chunk's columns in
+    // order.  A chunk lies with two warps (parts 0, 1 or 2, 3), so the running
+    // sum goes to and fro between them through shared memory, off the path of
+    // the GEMMs (the atom has been published), guarded by barriers.
+    const int pair = 4 * (part >> 1) + q;
+    uint32_t handed = 0;  // sums passed on by the even part so far
     float e_row = 0.f;  // ensemble-mean row energy, accumulated model by model in registers
     for (int it = 0; it < items.count && ok; ++it) {
+      // what the item is (worked out again for its last part, to hold fewer
+      // registers in between)
       int tile, m;
       items.at(it, tile, m);
-      // this CTA's models of the tile: [m_first, m_end)
-      const int m_first = max(0, items.lo - tile * M);
-      const int m_end = min(M, items.lo + items.count - tile * M);
-      const bool whole = m_first == 0 && m_end == M;
-      const bool last_here = m + 1 == m_end;
-      if (m == 0) e_row = 0.f;
-      const int tile_row = p.tile_row[tile];
-      const int g = m * p.n_species + p.tile_species[tile];
+      int g = m * p.n_species + p.tile_species[tile];
       // weight scales of this group (powers of two: the reciprocals are exact)
       float inv_s1 = 1.f, inv_s2 = 1.f, inv_s3 = 1.f, s_g = 1.f;
       if constexpr (F16) {
@@ -733,102 +756,116 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
         inv_s3 = 1.f / sc.z;
         s_g = sc.w;
       }
-      ok = __all_sync(0xffffffffu, wait_bar(&bars->bias_full, it & 1, abort_flag, p.err, p.timeout_ns));
-      if (!ok) break;
-      // E1: H1 = celu(Z1 + b1) -> act; celu'(z1) -> dc[0:d1]
-      if (!(ok = celu_layer(xpose, p.d1, 0, inv_s1, inv_s2))) break;
-      // E2: H2 = celu(Z2 + b2) -> act; celu'(z2) -> dc[d1:d1+d2]
-      if (!(ok = celu_layer(xpose + kBias, p.d2, p.d1, inv_s2, inv_s3))) break;
-      // E3: G3 = s_g w4 * celu'(z3) -> act, then, while B3 runs, the energy head:
-      // the part 0 and part 1 warps sum the 32-column chunks 0, 2, .. and
-      // 1, 3, .. of a row in column order (the accumulator still holds Z3), and
-      // the part 1 sum reaches the part 0 thread through shared memory guarded
-      // by two mbarriers (bounded waits, no CTA barrier).
+      const float dx_scale = p.inv_models * (inv_s1 / s_g);
+      const uint32_t R0 = lane_base, R1 = lane_base + 256;
+      if (!(ok = wait_all(&bars->bias_full, it & 1))) break;
+      // E1: H1 = celu(Z1 + b1); celu'(z1) -> dc[0:d1]
+      if (!(ok = celu_layer(R0, biases, p.d1, 0, inv_s1, inv_s2))) break;
+      // E2: H2 = celu(Z2 + b2); celu'(z2) -> dc[d1:d1+d2]
+      if (!(ok = celu_layer(R1, biases + kBias, p.d2, p.d1, inv_s2, inv_s3))) break;
+      // E3: G3 = s_g w4 * celu'(z3), and the energy head
       float e = 0.f;
       {
-        const uint32_t b = job & 1;
-        const float *bias = xpose + 2 * kBias, *w4 = xpose + 3 * kBias;
+        const float *bias = biases + 2 * kBias, *w4 = biases + 3 * kBias;
         const F2 isp = pack2(inv_s3, inv_s3), sgp = pack2(s_g, s_g);
-        if (!(ok = take_acc(b))) break;
-        if (grad) {
+        if (!(ok = take_acc())) break;
+        const int na = p.d3 / 64;
+        // the warp's staging tile holds H3 until the sum gets to it
+        float4* h3 = reinterpret_cast<float4*>(xpose + (warp - 2) * 32 * kGroup) + lane;
+        if (lane == 0) bulk_wait_read();
+        __syncwarp();
 #pragma unroll 1
-          for (int a = 0; a < p.d3 / 64; ++a) {
-            const int c = 64 * a + 16 * part;
-            float v[16];
-            tmem_ld16(tmem + b * 256 + lane_base + c, v);
+        for (int a = 0; a < na && ok; ++a) {
+          const int c = 64 * a + 16 * part;
+          float v[16];
+          tmem_ld16(R0 + c, v);
+          uint32_t w[16];
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              F2 bb[4], ww[4];
+          for (int k = 0; k < 4; ++k) {
+            F2 bb[2], ww[2], h[2];
+            load4(bias + c + 4 * k, bb[0], bb[1]);
+            load4(w4 + c + 4 * k, ww[0], ww[1]);
 #pragma unroll
-              for (int k = 0; k < 2; ++k) {
-                load4(bias + c + 8 * hf + 4 * k, bb[2 * k], bb[2 * k + 1]);
-                load4(w4 + c + 8 * hf + 4 * k, ww[2 * k], ww[2 * k + 1]);
-              }
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                ww[k] = mul2(mul2(sgp, ww[k]),
-                             dcelu2(fma2(pack2(v[8 * hf + 2 * k], v[8 * hf + 2 * k + 1]), isp, bb[k]), k2p));
-              act_store<F16>(act, r, c + 8 * hf, ww, grad_lo);
+            for (int u = 0; u < 2; ++u) {
+              F2 dh;
+              celu_pair2(fma2(pack2(v[4 * k + 2 * u], v[4 * k + 2 * u + 1]), isp, bb[u]), alp, nalp, k2p, h[u], dh);
+              split_pair<F16>(mul2(mul2(sgp, ww[u]), dh), g_lo, w[2 * k + u], w[8 + 2 * k + u]);
             }
+            float4 t;
+            unpack2(h[0], t.x, t.y);
+            unpack2(h[1], t.z, t.w);
+            h3[32 * k] = t;
+          }
+          if (grad) {
+            if constexpr (g_lo)
+              tmem_st16(R0 + c, w);
+            else
+              tmem_st8(R0 + c, w);
             publish_atom(a);
           }
-        }
-        if (part < 2) {
-#pragma unroll 1
-          for (int c = 32 * part; c < p.d3; c += 64) {
-#pragma unroll 1
-            for (int hh = 0; hh < 2; ++hh) {
-              float v[16];
-              tmem_ld16(tmem + b * 256 + lane_base + c + 16 * hh, v);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                F2 bb[2], ww[2];
-                load4(bias + c + 16 * hh + 4 * k, bb[0], bb[1]);
-                load4(w4 + c + 16 * hh + 4 * k, ww[0], ww[1]);
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                  F2 h, dh;
-                  celu_pair2(fma2(pack2(v[4 * k + 2 * u], v[4 * k + 2 * u + 1]), isp, bb[u]), alp, nalp, k2p, h, dh);
-                  float h0, h1, w0, w1;
-                  unpack2(h, h0, h1);
-                  unpack2(ww[u], w0, w1);
-                  e = fmaf(h0, w0, e);
-                  e = fmaf(h1, w1, e);
-                }
-              }
-            }
+          // the running sum of this warp's rows, on from the other warp's
+          if (part & 1) {
+            if (!(ok = wait_all(&bars->e_fwd[pair], handed & 1))) break;
+            e = bars->e_row[0][part >> 1][r];
+          } else if (a > 0) {
+            if (!(ok = wait_all(&bars->e_back[pair], (handed - 1) & 1))) break;
+            e = bars->e_row[1][part >> 1][r];
           }
-        }
-        release_acc(b);
-        if (part == 1) {
-          // the previous row energies must have been read before they are overwritten
-          if (it > 0) {
-            ok = __all_sync(0xffffffffu, wait_bar(&bars->ex_free, (it - 1) & 1, abort_flag, p.err, p.timeout_ns));
-            if (!ok) break;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 t = *reinterpret_cast<const float4*>(w4 + c + 4 * k), h = h3[32 * k];
+            e = fmaf(h.x, t.x, e);
+            e = fmaf(h.y, t.y, e);
+            e = fmaf(h.z, t.z, e);
+            e = fmaf(h.w, t.w, e);
           }
-          bars->ex[r] = e;
-          mbar_arrive(&bars->ex_ready);
+          if (!(part & 1)) {
+            bars->e_row[0][part >> 1][r] = e;
+            arrive(&bars->e_fwd[pair]);
+          } else {
+            // after the last atom nobody waits: the phase only keeps step
+            bars->e_row[1][part >> 1][r] = e;
+            arrive(&bars->e_back[pair]);
+          }
+          ++handed;
+        }
+        if (!ok) break;
+        if (!grad) {
+          fence_before_sync();
+          arrive(&bars->r0_free);
+        }
+        // the biases' place is free again
+        arrive(&bars->bias_free);
+        if (part == 3) {
+          bars->e_row[2][0][r] = e;
+          arrive(&bars->e_half[q]);
         }
       }
       if (grad) {
-        // E4: G2 = D2 * celu'(z2) -> act
-        if (!(ok = mask_layer(p.d2, p.d1))) break;
-        // E5: G1 = D1 * celu'(z1) -> act
-        if (!(ok = mask_layer(p.d1, 0))) break;
+        // E4: G2 = D2 * celu'(z2)
+        if (!(ok = mask_layer(R1, p.d2, p.d1))) break;
+        // E5: G1 = D1 * celu'(z1)
+        if (!(ok = mask_layer(R0, p.d1, 0))) break;
       }
-      // the row's energy
-      if (part == 0) {
-        ok = __all_sync(0xffffffffu, wait_bar(&bars->ex_ready, it & 1, abort_flag, p.err, p.timeout_ns));
-        if (!ok) break;
-        e += bars->ex[r] + __ldg(p.b4 + g);
-        mbar_arrive(&bars->ex_free);
-      }
-      if (part == 0) {
+      items.at(it, tile, m);
+      g = m * p.n_species + p.tile_species[tile];
+      const int tile_row = p.tile_row[tile];
+      const bool whole = it < items.nwhole || M == 1;
+      const int k = it - items.nwhole;  // among the CTA's items of shared tiles
+      // first model of the sum this one belongs to, and the sum's slot
+      const int first_shared = max(0, items.lo - (tile - items.shared0) * M);
+      const int m_first = whole ? 0 : (p.apart ? m : first_shared);
+      const int slot = whole ? 0 : (p.apart ? k : (tile == items.shared0 + items.lo / M ? 0 : 1));
+      const bool last_here = m + 1 == M;
+      // the row's energy (part 1 holds the first sum, part 3 the second)
+      if (part == 1) {
+        if (!(ok = wait_all(&bars->e_half[q], it & 1))) break;
+        e += bars->e_row[2][0][r] + __ldg(p.b4 + g);
         if (whole) {
-          e_row = fmaf(e, p.inv_models, e_row);
+          e_row = fmaf(e, p.inv_models, m == 0 ? 0.f : e_row);
           if (last_here) p.e_rows[tile_row + r] = e_row;
         } else {
-          p.e_part[((size_t)tile * M + m) * BM + r] = e;
+          p.e_part[(size_t)(items.lo + k) * BM + r] = e;
         }
       }
       // E6: dX groups.  A thread adds its 16 columns of a group to the models
@@ -838,13 +875,14 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
       // map, and the TMA engine writes it out.
       uint8_t* stage = reinterpret_cast<uint8_t*>(xpose + (warp - 2) * 32 * kGroup);
       uint8_t* trow = stage + lane * 64;
-      const float dx_scale = p.inv_models * (inv_s1 / s_g);
       const F2 dxs = pack2(dx_scale, dx_scale);
       const bool out = whole && last_here;
-      float4* sums = xs + (tile == items.lo / M ? 0 : (size_t)BM * p.d0 / 4);
-      for (int r0 = 0; r0 < p.ndx && ok; r0 += 16) {
-        const uint32_t b = job & 1;
-        const int ng = min(16, p.ndx - r0);
+      // laid out as the CELU' scratch
+      float4* sums = reinterpret_cast<float4*>(p.xs) +
+                     ((size_t)blockIdx.x * p.xs_slots + slot) * ((size_t)p.ndx * 4 * BM) + r;
+      for (int r0 = 0; r0 < p.ndx && ok; r0 += kRunGroups) {
+        const int ng = min(kRunGroups, p.ndx - r0);
+        const uint32_t at = R1 + 128 * (runs & 1);
 #pragma unroll 1
         for (int i = part; i < ng || i == part; i += 4) {
           float4 sum[4];
@@ -853,10 +891,10 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
 #pragma unroll
             for (int j = 0; j < 4; ++j) sum[j] = __ldcg(scratch + j * BM);
           }
-          if (i == part && !(ok = take_acc(b))) break;
+          if (i == part && !(ok = take_acc())) break;
           if (i >= ng) break;
           float v[16];
-          tmem_ld16(tmem + b * 256 + lane_base + i * kGroup, v);
+          tmem_ld16(at + i * kGroup, v);
           if (out) {
             if (lane == 0) bulk_wait_read();  // the tile's previous copy has read it
             __syncwarp();
@@ -886,13 +924,9 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
           }
         }
         if (!ok) break;
-        release_acc(b);
-      }
-      if (!ok) break;
-      // the biases' place is free again
-      if (lane == 0) {
-        bulk_wait_read();
-        mbar_arrive(&bars->bias_free);
+        fence_before_sync();
+        arrive(&bars->dx_free[runs & 1]);
+        ++runs;
       }
     }
     // the dX copies have completed (and no longer read shared memory) before
@@ -908,58 +942,61 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
   }
 }
 
-// Tiles whose models several CTAs of k_mlp_fused shared: dX and the energies of
-// the parts, added in model order.  Block (b, y): the tile that range b + 1
-// starts inside of, if no earlier range does; y: a dX column group, a thread
-// four columns of a row (four consecutive threads hold a row's 16).  It is
-// bound by latency (one round of loads per four parts): a block per group keeps
-// it to a few microseconds where one block per eight groups, a part after the
-// other, took 104 us on 192 atoms x 8 models.
+// The tiles left over: dX and the energies of their models, which several CTAs
+// of k_mlp_fused had, added in model order (or part by part, see apart).  Block
+// (t, y): a tile and a dX column group, a thread four columns of a row (four
+// consecutive threads hold a row's 16).  Bound by latency (a round of loads per
+// eight models): a block per group keeps it to a few microseconds where one
+// block per eight groups, a part after the other, took 104 us on 192 atoms x 8
+// models; with every column wanted by its memory traffic.
 constexpr int kJoinThreads = BM * 4;
 __global__ void __launch_bounds__(kJoinThreads) k_mlp_join(const __grid_constant__ FusedParams p, int blocks) {
   pdl_wait();
-  const int M = p.n_models, b = blockIdx.x + 1;
-  const int start = first_item(p.ntiles, M, b, blocks);
-  const int tile = start / M, t0 = tile * M;
-  if (start == t0 || first_item(p.ntiles, M, b - 1, blocks) > t0) return;  // no tile is cut here, or not first
-  const int row0 = p.tile_row[tile];
+  const int M = p.n_models, t0 = blockIdx.x * M;
+  const Share share(p.ntiles, M, blocks);
+  const int row0 = p.tile_row[share.whole * blocks + blockIdx.x];
   if (blockIdx.y == 0 && threadIdx.x < BM) {
     float e = 0.f;
-    const float* part = p.e_part + (size_t)tile * M * BM + threadIdx.x;
+    const float* part = p.e_part + (size_t)t0 * BM + threadIdx.x;
 #pragma unroll 4
     for (int m = 0; m < M; ++m) e = fmaf(__ldcg(part + (size_t)m * BM), p.inv_models, e);
     p.e_rows[row0 + threadIdx.x] = e;
   }
   const int i = blockIdx.y, r = threadIdx.x >> 2, j = threadIdx.x & 3;
   if (i >= p.ndx) return;
-  // part c of the tile lies in range c's first (slot 0) or another (slot 1) tile
   const float4* xs = reinterpret_cast<const float4*>(p.xs) + (size_t)(i * 4 + j) * BM + r;
-  const size_t per = (size_t)BM * p.d0 / 4;
-  float4 v;
-  for (int c0 = b - 1; c0 < blocks; c0 += 4) {
-    float4 t[4];
-    int n = 0;
+  const size_t per = (size_t)p.ndx * 4 * BM;
+  // slot of the k-th summand: model k, or part k (the CTAs from the tile's first on)
+  const int c0 = share.owner(t0);
+  const int n = p.apart ? M : share.owner(t0 + M - 1) - c0 + 1;
+  __shared__ int slots[kJoinThreads];
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < n; k0 += kJoinThreads) {
+    const int k = k0 + threadIdx.x;
+    __syncthreads();
+    if (k < n) {
+      const int c = p.apart ? share.owner(t0 + k) : c0 + k;
+      slots[threadIdx.x] = c * p.xs_slots + (p.apart ? t0 + k - share.first(c) : (share.first(c) / M == (int)blockIdx.x ? 0 : 1));
+    }
+    __syncthreads();
+    for (int u0 = 0; u0 < min(n - k0, kJoinThreads); u0 += 8) {
+      float4 t[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int lo = first_item(p.ntiles, M, c0 + k, blocks);
-      if (c0 + k < blocks && lo < t0 + M) {
-        t[k] = __ldcg(xs + ((size_t)(c0 + k) * 2 + (lo / M == tile ? 0 : 1)) * per);
-        n = k + 1;
+      for (int u = 0; u < 8; ++u)
+        if (k0 + u0 + u < n) t[u] = __ldcg(xs + (size_t)slots[u0 + u] * per);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (k0 + u0 + u >= n) break;
+        if (k0 + u0 + u == 0) {
+          v = t[0];
+        } else {
+          v.x += t[u].x;
+          v.y += t[u].y;
+          v.z += t[u].z;
+          v.w += t[u].w;
+        }
       }
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k >= n) break;
-      if (c0 + k == b - 1) {
-        v = t[k];
-      } else {
-        v.x += t[k].x;
-        v.y += t[k].y;
-        v.z += t[k].z;
-        v.w += t[k].w;
-      }
-    }
-    if (n < 4) break;
   }
   *reinterpret_cast<float4*>(p.dx + (size_t)(row0 + r) * p.d0 + p.dgroup[i] * kGroup + 4 * j) = v;
 }
@@ -1047,8 +1084,22 @@ int fused_grid(int tiles, int n_models) {
 size_t dc_bytes(int grid, const fennol_mlp_weights* w) {
   return (size_t)grid * BM * (w->dims[1] + w->dims[2]) * sizeof(float);
 }
-size_t xs_bytes(int grid, const fennol_mlp_weights* w) {
-  return w->n_models > 1 ? (size_t)grid * 2 * BM * w->dims[0] * sizeof(float) : 0;
+// Up to 16 dX column groups the models of a shared tile are kept apart, so that
+// its sum does not depend on how it was shared; wider rows are summed part by
+// part (kept apart, 256 molecules x 8 models would move 0.23 GB more).
+constexpr int kApartGroups = 16;
+int xs_slots(const Share& share, int ndx, int n_models) {
+  if (n_models == 1) return 0;
+  return std::max(1, ndx <= kApartGroups ? share.most() : std::min(share.most(), 2));
+}
+// for any number of tiles up to `tiles`
+size_t xs_bytes(int tiles, int grid, const fennol_mlp_weights* w) {
+  const int M = w->n_models;
+  if (M == 1 || grid == 0) return 0;
+  const size_t most = tiles < sm_count() ? ((size_t)tiles * M + grid - 1) / grid : M;
+  const size_t all = w->dims[0] / kGroup;
+  const size_t slots = std::max(std::min(most, (size_t)2) * all, most * std::min(all, (size_t)kApartGroups));
+  return (size_t)grid * slots * kGroup * BM * sizeof(float);
 }
 size_t e_part_bytes(int tiles, const fennol_mlp_weights* w) {
   return w->n_models > 1 ? (size_t)tiles * w->n_models * BM * sizeof(float) : 0;
@@ -1060,7 +1111,7 @@ size_t e_part_bytes(int tiles, const fennol_mlp_weights* w) {
 // whole), dX sums and energies of ensembles
 size_t fnl_mlp_fused_workspace(int rows, const fennol_mlp_weights* w) {
   const int grid = fused_grid(rows / BM, w->n_models);
-  return 256 + 128 + dc_bytes(grid, w) + xs_bytes(grid, w) + e_part_bytes(rows / BM, w);
+  return 256 + 128 + dc_bytes(grid, w) + xs_bytes(rows / BM, grid, w) + e_part_bytes(rows / BM, w);
 }
 
 int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
@@ -1072,58 +1123,57 @@ int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, 
   const int G = w->n_models * w->n_species;
   const bool f16 = is_f16_form(precision);
   const bool alo = precision == FENNOL_MLP_BF16X2 || f16;
-  const bool glo = precision == FENNOL_MLP_BF16X2;
   const bool wflo = f16;
   const bool wblo = precision == FENNOL_MLP_F16X3X2;
   if (f16 && (!w->wt_lo[0] || !w->wt_lo[1] || !w->wt_lo[2])) return FENNOL_ERR_INVALID;
   if (wblo && (!w->w_lo[0] || !w->w_lo[1] || !w->w_lo[2])) return FENNOL_ERR_INVALID;
   if (f16 && ((uintptr_t)w->f16_scale & 15) != 0) return FENNOL_ERR_INVALID;
   FusedParams p{};
-  // Column lists.  L1 streams units of 64 columns, or of 32 where that leaves
-  // out enough zero columns (a 32-column unit is half a 128-byte swizzle row:
-  // the same bytes in twice the copies).
+  // Column lists: the L1 units with a column that may be non-zero, and which of
+  // their K steps have one
   const int ngroups = d[0] / kGroup;
-  int n64 = 0, n32 = 0;
-  for (int c = 0; c < d[0] / 64; ++c) {
-    const bool h0 = xg.has(4 * c) || xg.has(4 * c + 1), h1 = xg.has(4 * c + 2) || xg.has(4 * c + 3);
-    n64 += h0 || h1;
-    n32 += (int)h0 + (int)h1;
-  }
-  if (n64 == 0) return FENNOL_ERR_INVALID;
-  p.unit = n32 * 5 <= n64 * 8 ? 32 : 64;
-  const int per = p.unit / kGroup;
-  for (int u = 0; u < ngroups / per; ++u) {
-    int bits = 0;
-    for (int k = 0; k < per; ++k) bits |= xg.has(u * per + k) ? 1 << k : 0;
+  for (int u = 0; u < ngroups / 2; ++u) {
+    const int bits = (xg.has(2 * u) ? 1 : 0) | (xg.has(2 * u + 1) ? 2 : 0);
     if (!bits) continue;
     p.xunit[p.nunits] = (unsigned char)u;
     p.xbits[p.nunits] = (unsigned char)bits;
     ++p.nunits;
   }
+  if (p.nunits == 0) return FENNOL_ERR_INVALID;
   if (dx)
     for (int g = 0; g < ngroups; ++g)
       if (dg.has(g)) p.dgroup[p.ndx++] = (unsigned char)g;
+  for (int i = 0, b = 0; i < p.ndx; ++b) {
+    const int left = std::min(kRunGroups - i % kRunGroups, p.ndx - i);
+    int n = 1;
+    while (n < left && n < 4 && p.dgroup[i + n] == p.dgroup[i] + n) ++n;
+    if (n == 3) n = 2;
+    p.box_g[b] = p.dgroup[i];
+    p.box_n[b] = (unsigned char)n;
+    i += n;
+  }
   // maps of absent low parts alias the high parts (never loaded)
   const void* wtl[3] = {wflo ? w->wt_lo[0] : w->wt_hi[0], wflo ? w->wt_lo[1] : w->wt_hi[1],
                         wflo ? w->wt_lo[2] : w->wt_hi[2]};
   const void* wl[3] = {wblo ? w->w_lo[0] : w->w_hi[0], wblo ? w->w_lo[1] : w->w_hi[1],
                        wblo ? w->w_lo[2] : w->w_hi[2]};
   Maps maps;
-  const uint32_t un = (uint32_t)p.unit;
-  bool ok = map2d(&maps.x, x, rows, d[0], BM, f16, un) && map2d(&maps.xlo, alo ? x_lo : x, rows, d[0], BM, f16, un) &&
-            map2d(&maps.w1t, w->wt_hi[0], (uint64_t)G * d[1], d[0], d[1], f16, un) &&
-            map2d(&maps.w1t_lo, wtl[0], (uint64_t)G * d[1], d[0], d[1], f16, un) &&
+  bool ok = map2d(&maps.x, x, rows, d[0], BM, f16, kUnit) && map2d(&maps.xlo, alo ? x_lo : x, rows, d[0], BM, f16, kUnit) &&
+            map2d(&maps.w1t, w->wt_hi[0], (uint64_t)G * d[1], d[0], d[1], f16, kUnit) &&
+            map2d(&maps.w1t_lo, wtl[0], (uint64_t)G * d[1], d[0], d[1], f16, kUnit) &&
             map2d(&maps.w2t, w->wt_hi[1], (uint64_t)G * d[2], d[1], d[2], f16) &&
             map2d(&maps.w3t, w->wt_hi[2], (uint64_t)G * d[3], d[2], d[3], f16) &&
             map2d(&maps.w3, w->w_hi[2], (uint64_t)G * d[2], d[3], d[2], f16) &&
             map2d(&maps.w2, w->w_hi[1], (uint64_t)G * d[1], d[2], d[1], f16) &&
             map2d(&maps.w1, w->w_hi[0], (uint64_t)G * d[0], d[1], 64, f16) &&
+            map2d(&maps.w1p, w->w_hi[0], (uint64_t)G * d[0], d[1], 2 * kGroup, f16) &&
             map2d(&maps.w1g, w->w_hi[0], (uint64_t)G * d[0], d[1], kGroup, f16) &&
             map2d(&maps.w2t_lo, wtl[1], (uint64_t)G * d[2], d[1], d[2], f16) &&
             map2d(&maps.w3t_lo, wtl[2], (uint64_t)G * d[3], d[2], d[3], f16) &&
             map2d(&maps.w3_lo, wl[2], (uint64_t)G * d[2], d[3], d[2], f16) &&
             map2d(&maps.w2_lo, wl[1], (uint64_t)G * d[1], d[2], d[1], f16) &&
             map2d(&maps.w1_lo, wl[0], (uint64_t)G * d[0], d[1], 64, f16) &&
+            map2d(&maps.w1p_lo, wl[0], (uint64_t)G * d[0], d[1], 2 * kGroup, f16) &&
             map2d(&maps.w1g_lo, wl[0], (uint64_t)G * d[0], d[1], kGroup, f16);
   if (ok && dx) ok = map_dx(&maps.dx, dx, rows, d[0]);
   if (!dx) maps.dx = maps.x;  // never used
@@ -1137,27 +1187,7 @@ int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, 
   p.d1 = d[1];
   p.d2 = d[2];
   p.d3 = d[3];
-  p.a_lo = alo ? 1 : 0;
-  p.g_lo = glo ? 1 : 0;
-  p.wf_lo = wflo ? 1 : 0;
   p.wb_lo = wblo ? 1 : 0;
-  p.bslots = glo ? 2 : kWSlots;
-  p.xstage = (uint32_t)p.unit * 2 * (2 * BM + 256 * (1 + p.wf_lo));
-  p.xstages = (int)(kRing / p.xstage);
-  // what each L1 stage lies on: per component (start, bytes), round the ring
-  for (int s = 0; s < p.xstages; ++s)
-    for (uint32_t off = 0; off < p.xstage; off += 8192) {  // every component is a multiple of 8 KB
-      const uint32_t a = (kXBase + s * p.xstage + off) % kRing;
-      if (a >= kActBytes) {
-        const int q = (int)((a - kActBytes) / kWStage);
-        p.stage_slots[s] |= 1u << q;
-        p.slot_stages[q] |= 1u << s;
-      } else if (a >= kActHalf && p.ndx > 0 && p.bslots == kWSlots) {
-        p.stage_slots[s] |= 4u << ((a - kActHalf) / kWStage);
-      } else {
-        p.stage_slots[s] |= 16u;
-      }
-    }
   p.scales = reinterpret_cast<const float4*>(w->f16_scale);
   p.alpha = w->celu_alpha;
   p.inv_models = 1.0f / (float)w->n_models;
@@ -1177,22 +1207,26 @@ int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, 
   }
   p.dc = (float*)(((uintptr_t)ws + 256 + 127) & ~(uintptr_t)127);
   const size_t smem = kSmemMain + sizeof(Bars) + 1024;
-  static bool attr[2] = {false, false};
-  auto kern = f16 ? k_mlp_fused<true> : k_mlp_fused<false>;
-  if (!attr[f16]) {
+  static bool attr[3] = {false, false, false};
+  const int form = f16 ? kF16 : (alo ? kBf16x2 : kBf16);
+  auto kern = form == kF16 ? k_mlp_fused<kF16> : (form == kBf16x2 ? k_mlp_fused<kBf16x2> : k_mlp_fused<kBf16>);
+  if (!attr[form]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return FENNOL_ERR_CUDA;
-    attr[f16] = true;
+    attr[form] = true;
   }
   if (ntiles <= 0) return FENNOL_OK;
   // one item per (tile, model); the CTAs share the items out evenly
   const int grid = fused_grid(ntiles, w->n_models);
   p.xs = (float*)((char*)p.dc + dc_bytes(grid, w));
-  p.e_part = (float*)((char*)p.xs + xs_bytes(grid, w));
+  p.e_part = (float*)((char*)p.xs + xs_bytes(ntiles, grid, w));
+  const Share share(ntiles, w->n_models, grid);
+  p.xs_slots = xs_slots(share, p.ndx, w->n_models);
+  p.apart = p.ndx <= kApartGroups;
   FNL_LAUNCH_PDL(kern, dim3(grid), dim3(kThreads), smem, st, maps, p);
   FNL_CHECK_LAUNCH();
-  if (w->n_models > 1 && ntiles % grid != 0) {  // ranges that begin inside a tile
-    FNL_LAUNCH_PDL(k_mlp_join, dim3(grid - 1, p.ndx > 0 ? p.ndx : 1), dim3(kJoinThreads), 0, st, p, grid);
+  if (w->n_models > 1 && share.left > 0) {
+    FNL_LAUNCH_PDL(k_mlp_join, dim3(share.left, p.ndx > 0 ? p.ndx : 1), dim3(kJoinThreads), 0, st, p, grid);
     FNL_CHECK_LAUNCH();
   }
   return FENNOL_OK;

@@ -171,16 +171,20 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr) {
   return d;
 }
 
-// The same for tiles of 32 16-bit elements (64 bytes) per row with 64-byte
-// swizzle: 8-row groups 512 bytes apart, layout type 4.
-__device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(512u >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)4 << 61;
-  return d;
+// The same in parts: the start address >> 4 (18-bit shared addresses), and the
+// high word of 64-element rows (128-byte swizzle) or of 32-element rows (64-byte
+// swizzle: 8-row groups 512 bytes apart, layout type 4).  A K step of 16 adds 2.
+__device__ __forceinline__ uint64_t sdesc_of(uint32_t addr16, uint32_t hi) {
+  return ((uint64_t)hi << 32) | (1u << 16) | (addr16 & 0x3FFFu);
+}
+__device__ __forceinline__ constexpr uint32_t sdesc_hi128() { return (1024u >> 4) | (1u << 14) | (2u << 29); }
+__device__ __forceinline__ constexpr uint32_t sdesc_hi64() { return (512u >> 4) | (1u << 14) | (4u << 29); }
+
+// True in one lane of the (converged) warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
 }
 
 // kind::f16 instruction descriptor: BF16 x BF16 -> F32, both K-major, M = 128.
@@ -199,6 +203,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same with the A operand in tensor memory: row i in lane i, 16 K elements
+// packed two to a column in 8 columns.
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -239,6 +254,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
   for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
+
+// 32 lanes x 16 (8) consecutive 32-bit columns per warp, from registers.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+          taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 }  // namespace umma
 }  // namespace fnl
