@@ -22,7 +22,14 @@ using namespace fnl;
 
 namespace {
 
-constexpr int kAevWarps = 8;
+// Warps of a block, one centre each and independent of one another: a block's
+// slot is free again when its longest centre is done.  98,304 atoms of water,
+// forward / adjoint: 8 warps 412 / 460 us, 4 warps 388 / 445, 2 warps 395 / 439;
+// 12,288 atoms: 60.4 / 71.0, 55.4 / 67.5, 55.2 / 68.4.
+constexpr int kAevWarps = 4;
+// a row capacity is taken while the staging of this many warps fits kStageLimit
+constexpr int kLimitWarps = 8;
+constexpr size_t kStageLimit = 200 * 1024;
 constexpr int kMaxS = 8;
 constexpr int kMaxP = kMaxS * (kMaxS + 1) / 2;
 // Angular neighbours a centre's staging holds: the row capacity, at most
@@ -251,6 +258,56 @@ __device__ __forceinline__ float zeta_pow(float x, int n, float f) {
   return f != 0.f ? r * exp2f_approx_pos(f * __log2f(x)) : r;
 }
 
+// Two FP32 values in one 64-bit register, and the packed FP32 instructions
+// (each half is rounded as the scalar instruction rounds it).
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(F2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+// zeta_pow of two values
+template <int N>
+__device__ __forceinline__ F2 zeta_pow2(float x0, float x1, int n, float f) {
+  F2 r = pack2(1.f, 1.f), b = pack2(x0, x1);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {  // n < 64
+    const bool bit = N >= 0 ? ((N >> k) & 1) != 0 : ((n >> k) & 1) != 0;
+    if (bit) r = mul2(r, b);
+    if (N >= 0 && (N >> (k + 1)) == 0) break;
+    b = mul2(b, b);
+  }
+  if (f != 0.f) {
+    const float2 l = unpack2(mul2(pack2(f, f), pack2(__log2f(x0), __log2f(x1))));
+    r = mul2(r, pack2(exp2f_approx_pos(l.x), exp2f_approx_pos(l.y)));
+  }
+  const float2 q = unpack2(r);
+  return pack2(x0 <= 0.f ? 0.f : q.x, x1 <= 0.f ? 0.f : q.y);
+}
+
 // integer part of zeta - 1 for a compile-time integer part ZN of zeta
 __host__ __device__ constexpr int zn_minus1(int zn) { return zn >= 0 ? zn - 1 : -1; }
 
@@ -353,8 +410,29 @@ __device__ __forceinline__ void stage_row(const Stage& st, int* cntw, const floa
   __syncwarp();
 }
 
-// Triangular index t -> (a, b), 0 <= a < b < n, b-major.
+// Triangular index t -> (a, b), 0 <= a < b, b-major: (0,1) (0,2) (1,2) (0,3) ...
+// The first 496 (b < 32, up to 32 neighbours of a species) come from a table, one
+// load in place of a square root and two corrections.
+constexpr int kTriMax = 32 * 31 / 2;
+struct TriTable {
+  unsigned short ab[kTriMax];  // a | b << 8
+};
+constexpr TriTable make_tri() {
+  TriTable t{};
+  int k = 0;
+  for (int b = 1; b < 32; ++b)
+    for (int a = 0; a < b; ++a) t.ab[k++] = (unsigned short)(a | (b << 8));
+  return t;
+}
+__device__ const TriTable kTri = make_tri();
+
 __device__ __forceinline__ void tri_ab(int t, int& a, int& b) {
+  if (t < kTriMax) {
+    const int v = __ldg(&kTri.ab[t]);
+    a = v & 0xFF;
+    b = v >> 8;
+    return;
+  }
   int bb = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)t)) * 0.5f);
   while (bb * (bb - 1) / 2 > t) --bb;
   while ((bb + 1) * bb / 2 <= t) ++bb;
@@ -362,18 +440,24 @@ __device__ __forceinline__ void tri_ab(int t, int& a, int& b) {
   a = t - bb * (bb - 1) / 2;
 }
 
-// Diagonal order of the pairs a < b of n items: d = b - a = 1, 2, ...; inside a
-// diagonal a increases.  Consecutive t rarely share an item (atomics stay
-// nearly conflict-free).
+// Diagonal order of the pairs a < b of n items: b - a = 1, 2, ...; inside a
+// diagonal a increases.  Consecutive t rarely share an item.  Counted from the
+// end, the diagonal of r pairs is the r-th run of the triangular order: with
+// (c, r) of the pair T - 1 - t, a = r - 1 - c and b - a = n - r.
 __device__ __forceinline__ void diag_ab(int t, int n, int& a, int& b) {
-  float q = (float)(2 * n - 1);
-  int u = (int)((q - sqrtf(fmaxf(q * q - 8.0f * (float)t, 0.f))) * 0.5f);
-  auto start = [&](int uu) { return (uu * (2 * n - 1) - uu * uu) / 2; };
-  while (u > 0 && start(u) > t) --u;
-  while (start(u + 1) <= t) ++u;
-  a = t - start(u);
-  b = a + u + 1;
+  int c, r;
+  tri_ab(n * (n - 1) / 2 - 1 - t, c, r);
+  a = r - 1 - c;
+  b = n - 1 - c;
 }
+
+// The 16-column groups of a row that the forward writes (bit g % 32 of w[g / 32]);
+// rows wider than the words hold are written whole (all).
+constexpr int kRowWords = 8;
+struct RowGroups {
+  unsigned w[kRowWords];
+  int all;
+};
 
 // q = floor(v / n), r = v - q n for 0 <= v < 2^16 and 1 <= n <= 256, from a
 // float reciprocal rn = 1/n: (v + 1/2) / n lies at least 1/(2n) from an
@@ -404,6 +488,23 @@ __device__ __forceinline__ float transpose_reduce32(float* v, int lane) {
     }
   }
   return v[0];
+}
+
+// The same of packed pairs: v[k] holds values 2k and 2k + 1.
+__device__ __forceinline__ float transpose_reduce32(F2* v, int lane) {
+#pragma unroll
+  for (int w = 16; w >= 2; w >>= 1) {
+    const bool upper = (lane & w) != 0;
+#pragma unroll
+    for (int k = 0; k < w / 2; ++k) {
+      const F2 send = upper ? v[k] : v[k + w / 2];
+      const F2 keep = upper ? v[k + w / 2] : v[k];
+      const float2 q = unpack2(send);
+      v[k] = add2(keep, pack2(__shfl_xor_sync(0xffffffffu, q.x, w), __shfl_xor_sync(0xffffffffu, q.y, w)));
+    }
+  }
+  const float2 q = unpack2(v[0]);
+  return ((lane & 1) ? q.y : q.x) + __shfl_xor_sync(0xffffffffu, (lane & 1) ? q.x : q.y, 1);
 }
 
 __device__ __forceinline__ void store_feature(int out_kind, void* out, void* out_lo, size_t idx, float v) {
@@ -464,13 +565,22 @@ __device__ __forceinline__ void copy_stage_async(const Stage& dst, const char* d
   }
 }
 
+// Forward.  Bound by instruction issue (about 3,500 warp instructions per water
+// centre; memory traffic would take a quarter of the time), at 28 warps per SM:
+// 72 registers, where 64 spill and are slower.  So the row's zeros are wide stores
+// of the groups that a later kernel reads (8 of 63 in water), absent species are
+// skipped, the pairs of one species come from a table and those of two from an
+// exact float quotient, and the products, the sums over the triplets and their
+// reduction are packed two to an instruction.  98,304 atoms of water 418 -> 388
+// us, 12,288 atoms 62 -> 55.4.
 template <int RD, int AD, int AS, int ZN>
 __global__ void __launch_bounds__(kAevWarps * 32)
 k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ atom_sys,
               const float* __restrict__ sys_cell, const int* __restrict__ nbr_j,
               const unsigned* __restrict__ nbr_shift, const int* __restrict__ nbr_count, int cap,
               const AevConst K, const int* __restrict__ atom_row, int out_kind, void* __restrict__ out,
-              void* __restrict__ out_lo, int ld, int* status, char* __restrict__ stage_g) {
+              void* __restrict__ out_lo, int ld, int vec, const __grid_constant__ RowGroups rg, int* status,
+              char* __restrict__ stage_g) {
   pdl_wait();
   extern __shared__ __align__(16) char smem_c[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -508,11 +618,37 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
   }
   const size_t orow = (size_t)atom_row[i] * ld;
 
+  // ---- zeros, 32 bytes per lane and group (vec: rows 16-byte aligned), before
+  // any feature is stored: most blocks of a row are empty
+  const int FR = S * RD;
+  {
+    const bool two = out_kind == FENNOL_AEV_BF16X2 || out_kind == FENNOL_AEV_F16X2;
+    const int per = out_kind == FENNOL_AEV_F32 ? 4 : 2;  // 16-byte chunks per group; bytes per value
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    for (int g0 = 0; g0 * 16 < K.F; g0 += 32) {
+      const int g = g0 + lane;
+      if (g * 16 >= K.F || !(rg.all || (rg.w[(g0 >> 5) & (kRowWords - 1)] >> lane) & 1u)) continue;
+      if (vec) {
+        uint4* q = reinterpret_cast<uint4*>((char*)out + (orow + 16 * g) * per);
+        for (int k = 0; k < per; ++k) q[k] = z;
+        if (two) {
+          q = reinterpret_cast<uint4*>((char*)out_lo + (orow + 16 * g) * per);
+          q[0] = z;
+          q[1] = z;
+        }
+      } else {
+        for (int k = 0; k < 16; ++k) store_feature(out_kind, out, out_lo, orow + 16 * g + k, 0.f);
+      }
+    }
+  }
+  __syncwarp();
+
   // ---- radial: lane (r, h) accumulates feature r over the neighbours h, h+nh, ...
   constexpr int nh = 32 / RD;
   const int r_lane = lane % RD, h_lane = lane / RD;
   const float sr = K.shift_r[r_lane], eta_r = K.eta_r;
-  for (int s = 0; s < S; ++s) {
+  for (unsigned m = __ballot_sync(0xffffffffu, lane < S && cnt_r > 0); m; m &= m - 1) {
+    const int s = __ffs(m) - 1;
     const int ns = __shfl_sync(0xffffffffu, cnt_r, s);
     const int os = __shfl_sync(0xffffffffu, off_r, s);
     float acc = 0.f;
@@ -525,9 +661,7 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
     if (h_lane == 0) store_feature(out_kind, out, out_lo, orow + s * RD + r_lane, acc);
   }
 
-  // ---- angular: zero every species-pair block, then fill the present ones
-  const int FR = S * RD;
-  for (int col = lane; col < K.P * 32; col += 32) store_feature(out_kind, out, out_lo, orow + FR + col, 0.f);
+  // ---- angular: the present species-pair blocks
   const float c_ang = K.c_ang, eta_a = K.eta_a;
   const unsigned present = __ballot_sync(0xffffffffu, lane < S && cnt_a > 0);
   for (unsigned m1 = present; m1; m1 &= m1 - 1) {
@@ -542,9 +676,10 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
       if (o1 + n1 > st.capa || o2 + n2 > st.capa) T = 0;  // overflowing atom: reported above
       if (T == 0) continue;
       const int p = triu_pair(s1, s2, S);
-      float acc[32];
+      const float r2 = 1.0f / (float)n2;
+      F2 acc[16];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+      for (int k = 0; k < 16; ++k) acc[k] = pack2(0.f, 0.f);
       for (int t0 = 0; t0 < T; t0 += 32) {
         const int t = t0 + lane;
         if (t < T) {
@@ -554,26 +689,31 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
             a += o1;
             b += o1;
           } else {
-            a = o1 + t / n2;
-            b = o2 + t % n2;
+            div_small(t, n2, r2, a, b);
+            a += o1;
+            b += o2;
           }
           const float4 ua = st.au[a], ub = st.au[b];
           const float cosang = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
           const float ct = 0.95f * cosang;
           const float stt = sqrtf(fmaxf(1.0f - ct * ct, 0.f));
           const float f = c_ang * st.af[a].x * st.af[b].x;
-          float A[AS], B[AD];
+          F2 A[AS / 2];
+          float B[AD];
 #pragma unroll
-          for (int z = 0; z < AS; ++z) {
-            float cz = ct * K.cosz[z] + stt * K.sinz[z];
-            A[z] = f * zeta_pow<ZN>(1.0f + cz, K.zeta_n, K.zeta_f);
+          for (int z = 0; z < AS / 2; ++z) {
+            const float c0 = ct * K.cosz[2 * z] + stt * K.sinz[2 * z];
+            const float c1 = ct * K.cosz[2 * z + 1] + stt * K.sinz[2 * z + 1];
+            A[z] = mul2(pack2(f, f), zeta_pow2<ZN>(1.0f + c0, 1.0f + c1, K.zeta_n, K.zeta_f));
           }
           const float dm = 0.5f * (ua.w + ub.w);
           gauss_chain<AD>(dm - K.shift_a[0], eta_a, K.dra, K.gc2a, B);
 #pragma unroll
-          for (int r = 0; r < AD; ++r)
+          for (int r = 0; r < AD; ++r) {
+            const F2 b2 = pack2(B[r], B[r]);
 #pragma unroll
-            for (int z = 0; z < AS; ++z) acc[r * AS + z] = fmaf(A[z], B[r], acc[r * AS + z]);
+            for (int z = 0; z < AS / 2; ++z) acc[r * AS / 2 + z] = fma2(A[z], b2, acc[r * AS / 2 + z]);
+          }
         }
       }
       const float v = transpose_reduce32(acc, lane);
@@ -583,8 +723,31 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
   }
 }
 
+// Warp-collective: rows[slot] += (x, y, z) of every active lane, lanes of the same
+// slot one after the other in lane order.  Float atomics in shared memory are
+// compare-and-swap loops: on the triplets of a water centre they took 4.5 rounds
+// each, 134 per centre with a shared-memory round trip in every one; here a
+// round serves all three components of all lanes whose turn it is.
+__device__ __forceinline__ void add_rows(float4* rows, int slot, bool active, float x, float y, float z, int lane) {
+  const unsigned same = __match_any_sync(0xffffffffu, active ? slot : -1 - lane);
+  const int turn = __popc(same & ((1u << lane) - 1u));
+  const int turns = __reduce_max_sync(0xffffffffu, turn);
+  for (int k = 0; k <= turns; ++k) {
+    if (turn == k && active) {
+      float4 v = rows[slot];
+      v.x += x;
+      v.y += y;
+      v.z += z;
+      rows[slot] = v;
+    }
+    __syncwarp();
+  }
+}
+
 // --------------------------------------------------------------------------------
-// Adjoint: dE/dAEV -> forces.
+// Adjoint: dE/dAEV -> forces.  98,304 atoms of water 579 -> 445 us, 12,288 atoms
+// 90.6 -> 67.5 us: add_rows in place of shared float atomics (483 / 72.3), pairs from
+// the table (468 / 71), blocks of 4 warps.
 // --------------------------------------------------------------------------------
 constexpr int kMaxBlk = kMaxP;  // species-pair blocks of one centre atom
 
@@ -593,7 +756,7 @@ __host__ __device__ __forceinline__ size_t bwd_bytes(int S, int RD, int cap) {
 }
 
 template <int RD, int AD, int AS, int ZN, bool kVir, bool kStaged>
-__global__ void __launch_bounds__(kAevWarps * 32, 4)
+__global__ void __launch_bounds__(kAevWarps * 32, 32 / kAevWarps)
 k_aev_backward(const float4* __restrict__ xyzs, int n, const int* __restrict__ atom_sys,
                const float* __restrict__ sys_cell, const int* __restrict__ nbr_j,
                const unsigned* __restrict__ nbr_shift, const int* __restrict__ nbr_count, int cap,
@@ -610,7 +773,6 @@ k_aev_backward(const float4* __restrict__ xyzs, int n, const int* __restrict__ a
   Stage st = carve_stage(base, cap, false);
   // the edge vectors in st.tmp[k] are replaced by the gradient of the energy
   // with respect to edge k (x, y, z) once the radial pass has read them
-  float* gk = reinterpret_cast<float*>(st.tmp);
   float* gr = (float*)(base + stage_bytes(cap, false));               // [S][RD+1]
   int* blkw = (int*)(gr + S * (RD + 1));                              // block table
 
@@ -734,7 +896,9 @@ k_aev_backward(const float4* __restrict__ xyzs, int n, const int* __restrict__ a
   __syncwarp();
   const int nblk = blk_cum[kMaxBlk + 1];
   const int Ttot = blk_cum[nblk];
-  for (int t = lane; t < Ttot; t += 32) {
+  for (int t0 = 0; t0 < Ttot; t0 += 32) {
+    const bool active = t0 + lane < Ttot;
+    const int t = min(t0 + lane, Ttot - 1);
     int k = 0;
     while (k + 1 < nblk && blk_cum[k + 1] <= t) ++k;
     const int tl = t - blk_cum[k];
@@ -812,12 +976,10 @@ k_aev_backward(const float4* __restrict__ xyzs, int n, const int* __restrict__ a
     const float dEdc = cfab * Th * (-0.95f * rsqrtf(fmaxf(1.0f - ct * ct, 1e-12f)));
     const float ia = __fdividef(dEdc, ua.w), ib = __fdividef(dEdc, ub.w);
     const int sa_ = st.aslot[a], sb_ = st.aslot[b];
-    atomicAdd(gk + 4 * sa_, dEdda * ua.x + ia * (ub.x - cosang * ua.x));
-    atomicAdd(gk + 4 * sa_ + 1, dEdda * ua.y + ia * (ub.y - cosang * ua.y));
-    atomicAdd(gk + 4 * sa_ + 2, dEdda * ua.z + ia * (ub.z - cosang * ua.z));
-    atomicAdd(gk + 4 * sb_, dEddb * ub.x + ib * (ua.x - cosang * ub.x));
-    atomicAdd(gk + 4 * sb_ + 1, dEddb * ub.y + ib * (ua.y - cosang * ub.y));
-    atomicAdd(gk + 4 * sb_ + 2, dEddb * ub.z + ib * (ua.z - cosang * ub.z));
+    add_rows(st.tmp, sa_, active, dEdda * ua.x + ia * (ub.x - cosang * ua.x),
+             dEdda * ua.y + ia * (ub.y - cosang * ua.y), dEdda * ua.z + ia * (ub.z - cosang * ua.z), lane);
+    add_rows(st.tmp, sb_, active, dEddb * ub.x + ib * (ua.x - cosang * ub.x),
+             dEddb * ub.y + ib * (ua.y - cosang * ub.y), dEddb * ub.z + ib * (ua.z - cosang * ub.z), lane);
   }
   __syncwarp();
 
@@ -848,7 +1010,14 @@ k_aev_backward(const float4* __restrict__ xyzs, int n, const int* __restrict__ a
     for (int k = lane; k < cnt; k += 32) {
       const float4 gv = st.tmp[k];
       float rx, ry, rz;
-      edge_vec(pi, xyzs[__ldg(nbr_j + row + k)], __ldg(nbr_shift + row + k), c, rx, ry, rz);
+      if constexpr (kStaged) {
+        const float4 e = __ldg(in_record(rec, base, st.tmp) + k);
+        rx = e.x;
+        ry = e.y;
+        rz = e.z;
+      } else {
+        edge_vec(pi, xyzs[__ldg(nbr_j + row + k)], __ldg(nbr_shift + row + k), c, rx, ry, rz);
+      }
       v[0] = fmaf(rx, gv.x, v[0]);
       v[1] = fmaf(rx, gv.y, v[1]);
       v[2] = fmaf(rx, gv.z, v[2]);
@@ -964,6 +1133,7 @@ k_aev_tangent(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
       if (o1 + n1 > st.capa || o2 + n2 > st.capa) T = 0;
       if (T == 0) continue;
       const int p = triu_pair(s1, s2, S);
+      const float r2 = 1.0f / (float)n2;
       float acc[32];
 #pragma unroll
       for (int k = 0; k < 32; ++k) acc[k] = 0.f;
@@ -976,8 +1146,9 @@ k_aev_tangent(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
             a += o1;
             b += o1;
           } else {
-            a = o1 + t / n2;
-            b = o2 + t % n2;
+            div_small(t, n2, r2, a, b);
+            a += o1;
+            b += o2;
           }
           const float4 ua = st.au[a], ub = st.au[b];
           const float2 fa = st.af[a], fb = st.af[b];
@@ -1036,6 +1207,7 @@ struct AevKernels {
   static constexpr auto bwd = k_aev_backward<RD, AD, AS, ZN, false, false>;
   static constexpr auto bwdv = k_aev_backward<RD, AD, AS, ZN, true, false>;
   static constexpr auto bwds = k_aev_backward<RD, AD, AS, ZN, false, true>;
+  static constexpr auto bwdvs = k_aev_backward<RD, AD, AS, ZN, true, true>;
   static constexpr auto tan = k_aev_tangent<RD, AD, AS, ZN>;
 };
 
@@ -1130,7 +1302,8 @@ extern "C" int fennol_pack_atoms(const float* coords, const int* species_idx, in
 static int aev_forward_launch(const float* xyzs, int natoms, const int* atom_sys, const float* sys_cell,
                               const int* nbr_j, const unsigned* nbr_shift, const int* nbr_count, int capacity,
                               const fennol_aev_params* p, const int* atom_row, int out_kind, void* out,
-                              void* out_lo, int ld, int* status, void* stage, void* stream) {
+                              void* out_lo, int ld, const unsigned long long* groups, int words, int* status,
+                              void* stage, void* stream) {
   AevConst K;
   if (!make_const(p, &K)) return FENNOL_ERR_UNSUPPORTED;
   if (natoms < 0 || capacity <= 0 || ld < K.F) return FENNOL_ERR_INVALID;
@@ -1141,14 +1314,19 @@ static int aev_forward_launch(const float* xyzs, int natoms, const int* atom_sys
       out_kind != FENNOL_AEV_F16X2)
     return FENNOL_ERR_INVALID;
   if ((out_kind == FENNOL_AEV_BF16X2 || out_kind == FENNOL_AEV_F16X2) && !out_lo) return FENNOL_ERR_INVALID;
-  if ((size_t)kAevWarps * stage_bytes(capacity) > 200 * 1024) return FENNOL_ERR_UNSUPPORTED;
+  if (kLimitWarps * stage_bytes(capacity) > kStageLimit) return FENNOL_ERR_UNSUPPORTED;
+  const int size = out_kind == FENNOL_AEV_F32 ? 4 : 2;
+  RowGroups rg = {};
+  rg.all = !groups || K.F > kRowWords * 32 * 16;
+  for (int k = 0; !rg.all && k < kRowWords && k / 2 < words; ++k) rg.w[k] = (unsigned)(groups[k / 2] >> (32 * (k & 1)));
+  const int vec = (((uintptr_t)out | (uintptr_t)out_lo) & 15) == 0 && (size_t)ld * size % 16 == 0;
   int blocks = (natoms + kAevWarps - 1) / kAevWarps;
   bool launched = dispatch(K, [&](auto ks) {
     size_t smem = set_smem((const void*)ks.fwd, (size_t)kAevWarps * stage_bytes(capacity));
     if (!smem) return false;
     if (launch_pdl(ks.fwd, blocks, kAevWarps * 32, smem, (cudaStream_t)stream, 
         (const float4*)xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, K,
-        atom_row, out_kind, out, out_lo, ld, status, (char*)stage) != cudaSuccess) return false;
+        atom_row, out_kind, out, out_lo, ld, vec, rg, status, (char*)stage) != cudaSuccess) return false;
     return true;
   });
   if (!launched) return FENNOL_ERR_UNSUPPORTED;
@@ -1162,7 +1340,7 @@ extern "C" int fennol_aev_forward(const float* xyzs, int natoms, const int* atom
                                   const int* atom_row, int out_kind, void* out, void* out_lo, int ld,
                                   int* status, void* stream) {
   return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
-                            out_kind, out, out_lo, ld, status, nullptr, stream);
+                            out_kind, out, out_lo, ld, nullptr, 0, status, nullptr, stream);
 }
 
 extern "C" size_t fennol_aev_stage_bytes(int natoms, int capacity) {
@@ -1178,7 +1356,20 @@ extern "C" int fennol_aev_forward_staged(const float* xyzs, int natoms, const in
   if (natoms > 0 && (!stage || ((uintptr_t)stage & 15) != 0)) return FENNOL_ERR_INVALID;
   if (stage_bytes_ < fennol_aev_stage_bytes(natoms, capacity)) return FENNOL_ERR_WORKSPACE;
   return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
-                            out_kind, out, out_lo, ld, status, stage, stream);
+                            out_kind, out, out_lo, ld, nullptr, 0, status, stage, stream);
+}
+
+extern "C" int fennol_aev_forward_groups(const float* xyzs, int natoms, const int* atom_sys,
+                                         const float* sys_cell, const int* nbr_j, const unsigned* nbr_shift,
+                                         const int* nbr_count, int capacity, const fennol_aev_params* p,
+                                         const int* atom_row, int out_kind, void* out, void* out_lo, int ld,
+                                         const unsigned long long* host_groups, int group_words, void* stage,
+                                         size_t stage_bytes_, int* status, void* stream) {
+  if (host_groups && (long long)group_words * 64 * 16 < fennol_aev_length(p)) return FENNOL_ERR_INVALID;
+  if (stage && ((uintptr_t)stage & 15) != 0) return FENNOL_ERR_INVALID;
+  if (stage && stage_bytes_ < fennol_aev_stage_bytes(natoms, capacity)) return FENNOL_ERR_WORKSPACE;
+  return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
+                            out_kind, out, out_lo, ld, host_groups, group_words, status, stage, stream);
 }
 
 static int aev_backward_launch(const float* xyzs, int natoms, const int* atom_sys, const float* sys_cell,
@@ -1195,10 +1386,10 @@ static int aev_backward_launch(const float* xyzs, int natoms, const int* atom_sy
   // the kernel reads dE/dAEV pair blocks as float4
   if ((ld & 3) != 0 || ((uintptr_t)daev & 15) != 0) return FENNOL_ERR_INVALID;
   size_t bytes = (size_t)kAevWarps * bwd_bytes(K.S, K.RD, capacity);
-  if (bytes > 200 * 1024) return FENNOL_ERR_UNSUPPORTED;
+  if (kLimitWarps * bwd_bytes(K.S, K.RD, capacity) > kStageLimit) return FENNOL_ERR_UNSUPPORTED;
   int blocks = (natoms + kAevWarps - 1) / kAevWarps;
   bool launched = dispatch(K, [&](auto ks) {
-    auto fn = atom_virial ? ks.bwdv : (stage ? ks.bwds : ks.bwd);
+    auto fn = atom_virial ? (stage ? ks.bwdvs : ks.bwdv) : (stage ? ks.bwds : ks.bwd);
     size_t smem = set_smem((const void*)fn, bytes);
     if (!smem) return false;
     if (launch_pdl(fn, blocks, kAevWarps * 32, smem, (cudaStream_t)stream, 
@@ -1240,6 +1431,17 @@ extern "C" int fennol_aev_backward_virial(const float* xyzs, int natoms, const i
                              atom_row, daev, ld, forces4, atom_virial, status, nullptr, stream);
 }
 
+extern "C" int fennol_aev_backward_virial_staged(const float* xyzs, int natoms, const int* atom_sys,
+                                                 const float* sys_cell, const int* nbr_j,
+                                                 const unsigned* nbr_shift, const int* nbr_count, int capacity,
+                                                 const fennol_aev_params* p, const int* atom_row,
+                                                 const float* daev, int ld, float* forces4, float* atom_virial,
+                                                 const void* stage, int* status, void* stream) {
+  if (natoms > 0 && (!atom_virial || !stage || ((uintptr_t)stage & 15) != 0)) return FENNOL_ERR_INVALID;
+  return aev_backward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p,
+                             atom_row, daev, ld, forces4, atom_virial, status, stage, stream);
+}
+
 extern "C" int fennol_aev_tangent(const float* xyzs, int natoms, const int* atom_sys,
                                   const float* sys_cell, const int* nbr_j, const unsigned* nbr_shift,
                                   const int* nbr_count, int capacity, const fennol_aev_params* p,
@@ -1252,7 +1454,7 @@ extern "C" int fennol_aev_tangent(const float* xyzs, int natoms, const int* atom
   if (!xyzs || !atom_sys || !nbr_j || !nbr_shift || !nbr_count || !atom_row || !du4 || !out)
     return FENNOL_ERR_INVALID;
   size_t bytes = (size_t)kAevWarps * jvp_bytes(capacity);
-  if (bytes > 200 * 1024) return FENNOL_ERR_UNSUPPORTED;
+  if (kLimitWarps * jvp_bytes(capacity) > kStageLimit) return FENNOL_ERR_UNSUPPORTED;
   int blocks = (natoms + kAevWarps - 1) / kAevWarps;
   bool launched = dispatch(K, [&](auto ks) {
     size_t smem = set_smem((const void*)ks.tan, bytes);

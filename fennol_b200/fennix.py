@@ -1117,7 +1117,7 @@ class FENNIX:
         call("fennol_pack_atoms", inputs["_coords"].data_ptr(), layout.t_species.data_ptr(), layout.n,
              ws.xyzs.data_ptr(), st)
         view = _RowsView(rows)
-        if want_forces and not want_virial:
+        if want_forces:
             view.aev_stage = self._stage_buffer(layout.n, rows.capacity)
         pot.launch_forces(layout, view, ws, st, want_forces, want_virial)
         # the outputs are enqueued before the status read, so that one host

@@ -531,20 +531,15 @@ class ANIPotential:
         lib_p = C_ptr(self.params)
         n = layout.n
         # the adjoint reuses the forward's staging when the buffers carry it
-        staged = want_forces and not want_virial and getattr(g, "aev_stage", None) is not None
-        if staged:
-            call("fennol_aev_forward_staged", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
-                 layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
-                 g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.aev_kind, ws.x.data_ptr(),
-                 _ptr(ws.x_lo), ws.x.shape[1], g.aev_stage.data_ptr(), g.aev_stage.numel(),
-                 ws.status.data_ptr(), stream)
-        else:
-            call("fennol_aev_forward", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
-                 layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
-                 g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.aev_kind, ws.x.data_ptr(),
-                 _ptr(ws.x_lo), ws.x.shape[1], ws.status.data_ptr(), stream)
-        # the columns that can be non-zero are also the ones the adjoint reads
+        stage = getattr(g, "aev_stage", None) if want_forces else None
+        # the columns that can be non-zero are the ones the forward writes (the
+        # workspace starts as zeros), the MLP reads and the adjoint reads
         groups = self.active_groups(layout.species_mask)
+        call("fennol_aev_forward_groups", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
+             layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
+             g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.aev_kind, ws.x.data_ptr(), _ptr(ws.x_lo),
+             ws.x.shape[1], groups.ctypes.data, groups.size, _ptr(stage), 0 if stage is None else stage.numel(),
+             ws.status.data_ptr(), stream)
         call("fennol_mlp_energy_grad_groups", self.precision, layout.rows, layout.ntiles,
              layout.t_tile_species.data_ptr(), layout.t_tile_row.data_ptr(), C_ptr(self.mlp.struct),
              ws.x.data_ptr(), _ptr(ws.x_lo), groups.ctypes.data, groups.ctypes.data, groups.size,
@@ -560,18 +555,22 @@ class ANIPotential:
         if want_forces and want_virial:
             ws.forces4.zero_()
             av, vir = ws.virial_buffers(layout)
-            call("fennol_aev_backward_virial", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
-                 layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
-                 g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1],
-                 ws.forces4.data_ptr(), av.data_ptr(), ws.status.data_ptr(), stream)
+            args = (ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(), layout.t_cell.data_ptr(),
+                    g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(), g.cap_r, lib_p,
+                    layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1], ws.forces4.data_ptr(),
+                    av.data_ptr())
+            if stage is not None:
+                call("fennol_aev_backward_virial_staged", *args, stage.data_ptr(), ws.status.data_ptr(), stream)
+            else:
+                call("fennol_aev_backward_virial", *args, ws.status.data_ptr(), stream)
             call("fennol_virial_reduce", av.data_ptr(), n, layout.t_sys_start.data_ptr(), layout.nsys,
                  float(self.unit_scale), vir.data_ptr(), stream)
-        elif staged:
+        elif stage is not None:
             ws.forces4.zero_()
             call("fennol_aev_backward_staged", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
                  layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
                  g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1],
-                 ws.forces4.data_ptr(), g.aev_stage.data_ptr(), ws.status.data_ptr(), stream)
+                 ws.forces4.data_ptr(), stage.data_ptr(), ws.status.data_ptr(), stream)
         elif want_forces:
             ws.forces4.zero_()
             call("fennol_aev_backward", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),

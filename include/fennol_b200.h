@@ -268,6 +268,22 @@ int fennol_aev_backward_staged(const float* xyzs, int natoms, const int* atom_sy
                                const void* stage, int* status, void* stream);
 
 /*
+ * The forward for rows of which only some columns are read: only the 16-column
+ * groups named in host_groups (host memory; bit g % 64 of host_groups[g / 64],
+ * group_words words that cover the row; NULL: all of them) are written, the
+ * other columns of out and out_lo stay as they are.  The caller names every
+ * group that can be non-zero (fennol_aev_active_groups for a species set);
+ * the features of a block outside them are stored all the same.  stage: NULL,
+ * or as for fennol_aev_forward_staged.
+ */
+int fennol_aev_forward_groups(const float* xyzs, int natoms, const int* atom_sys,
+                              const float* sys_cell, const int* nbr_j, const unsigned* nbr_shift,
+                              const int* nbr_count, int capacity, const fennol_aev_params* p,
+                              const int* atom_row, int out_kind, void* out, void* out_lo, int ld,
+                              const unsigned long long* host_groups, int group_words, void* stage,
+                              size_t stage_bytes, int* status, void* stream);
+
+/*
  * fennol_aev_backward that also writes, per centre atom i, the 3x3 sum over
  * its edges of r_ij (x) dE/dr_ij (atom_virial, float32 [natoms*9], row-major
  * a,b = r_a * g_b).  Summed per system (fennol_virial_reduce) this is the
@@ -279,6 +295,14 @@ int fennol_aev_backward_virial(const float* xyzs, int natoms, const int* atom_sy
                                const int* nbr_count, int capacity, const fennol_aev_params* p,
                                const int* atom_row, const float* daev, int ld, float* forces4,
                                float* atom_virial, int* status, void* stream);
+/* fennol_aev_backward_virial reading the staged neighbourhoods of the forward. */
+int fennol_aev_backward_virial_staged(const float* xyzs, int natoms, const int* atom_sys,
+                                      const float* sys_cell, const int* nbr_j,
+                                      const unsigned* nbr_shift, const int* nbr_count, int capacity,
+                                      const fennol_aev_params* p, const int* atom_row,
+                                      const float* daev, int ld, float* forces4, float* atom_virial,
+                                      const void* stage, int* status, void* stream);
+
 
 /*
  * Forward-mode tangent of the AEV: out[atom_row[i]*ld + f] = sum_k

@@ -140,3 +140,83 @@ def test_staged_adjoint_matches_unstaged(cuda_device):
     assert int(ws.status[_lib.ST_ANG_OVERFLOW]) == 0
     scale = np.abs(f[0]).max()
     np.testing.assert_allclose(f[1], f[0], atol=1e-5 * scale, rtol=0)
+
+
+@pytest.mark.parametrize("n_h,n_o", [(2, 1), (8, 1), (9, 3), (32, 2), (33, 1), (44, 6)])
+def test_crowded_centres_vs_fp64(pot32, n_h, n_o):
+    """Clusters in which every atom is an angular neighbour of every other: a
+    triplet count at and around multiples of 32, one and several species, more
+    neighbours of a species than the pair table holds (32), and rounds in
+    which most lanes add to the same neighbour.
+
+    Bound: a triplet's force terms carry about 2e-6 (the power of the angular
+    factor) plus the float32 rounding of the sums; up to 49 * 48 of them of
+    either sign meet in one force, whose sum of moduli is up to some 50 times
+    the largest force: 1e-4 of it."""
+    rng = np.random.default_rng(100 * n_h + n_o)
+    n = n_h + n_o
+    xyz = np.zeros((0, 3))
+    while len(xyz) < n:  # a ball of radius 1.7, no two atoms nearer than 0.55
+        p = rng.uniform(-1.7, 1.7, 3)
+        if p @ p < 1.7 ** 2 and (len(xyz) == 0 or np.linalg.norm(xyz - p, axis=1).min() > 0.55):
+            xyz = np.vstack([xyz, p])
+    sp = np.array([1] * n_h + [8] * n_o)[rng.permutation(n)]
+    xyz = xyz.astype(np.float32).astype(np.float64)
+    r = ani_ref.energy_and_forces(xyz, sp, [n], pot32.weights, CFG, MCFG)
+    _, f = pot32.energy_and_forces(xyz, sp, [n])
+    np.testing.assert_allclose(f.cpu().numpy(), r["forces"], rtol=0, atol=1e-4 * np.abs(r["forces"]).max())
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16", "bf16x2", "f16x3x1"])
+@pytest.mark.parametrize("off", [0, 1])
+def test_forward_groups_and_staged_virial(cuda_device, precision, off):
+    """fennol_aev_forward_groups writes the named column groups as
+    fennol_aev_forward does (also at an output off 16 bytes) and no others, and
+    the virial adjoint reads its staging: the same arithmetic in another
+    instantiation, so a few float32 roundings (1e-6) of the largest value; the
+    forces in the order of their atomics (1e-5, as above)."""
+    from fennol_b200 import _lib
+    from fennol_b200._lib import call
+    from fennol_b200.potential import C_ptr
+
+    pot = ANIPotential(precision=precision, device=cuda_device, seed=0)
+    s = water_box(5, seed=33)
+    x = torch.tensor(s.coordinates, dtype=torch.float32, device=cuda_device)
+    pot.energy_and_forces(x, s.species, [s.natoms], s.cell[None])
+    lay, g, ws = next(iter(pot._cache.values()))
+    st = torch.cuda.current_stream().cuda_stream
+    args = (ws.xyzs.data_ptr(), lay.n, lay.t_atom_sys.data_ptr(), lay.t_cell.data_ptr(), g.rad_j.data_ptr(),
+            g.rad_s.data_ptr(), g.rad_n.data_ptr(), g.cap_r, C_ptr(pot.params), lay.t_atom_row.data_ptr())
+    rows, d0 = ws.x.shape
+    F = pot.aev_cfg.aev_length
+    groups = pot.active_groups(lay.species_mask)
+    named = np.array([(int(groups[c // 1024]) >> (c // 16 % 64)) & 1 for c in range(F)], bool)
+    assert 0 < named.sum() < F
+    got = []
+    for words in (None, groups):
+        bufs = [torch.full((rows * d0 + off,), 7.0, dtype=ws.x.dtype, device=cuda_device) for _ in range(2)]
+        lo = bufs[1][off:] if ws.x_lo is not None else None
+        out = (ws.aev_kind, bufs[0][off:].data_ptr(), None if lo is None else lo.data_ptr(), d0)
+        if words is None:
+            call("fennol_aev_forward", *args, *out, ws.status.data_ptr(), st)
+        else:
+            call("fennol_aev_forward_groups", *args, *out, words.ctypes.data, words.size, g.aev_stage.data_ptr(),
+                 g.aev_stage.numel(), ws.status.data_ptr(), st)
+        got.append([b[off:].view(rows, d0)[lay.t_atom_row.long(), :F].float().cpu().numpy() for b in bufs])
+    for k, (full, part) in enumerate(zip(*got)):
+        np.testing.assert_array_equal(part[:, named], full[:, named])
+        assert (part[:, ~named] == 7.0).all()
+        assert k == 1 and ws.x_lo is None or (full[:, ~named] == 0.0).all()
+    ws.dx.normal_()  # any dE/dAEV rows
+    f, v = [], []
+    for name, extra in (("fennol_aev_backward_virial", ()),
+                        ("fennol_aev_backward_virial_staged", (g.aev_stage.data_ptr(),))):
+        ws.forces4.zero_()
+        av = torch.zeros((lay.n, 9), device=cuda_device)
+        call(name, *args, ws.dx.data_ptr(), ws.dx.shape[1], ws.forces4.data_ptr(), av.data_ptr(), *extra,
+             ws.status.data_ptr(), st)
+        f.append(ws.forces4[:lay.n, :3].cpu().numpy())
+        v.append(av.cpu().numpy())
+    assert int(ws.status[_lib.ST_ANG_OVERFLOW]) == 0
+    np.testing.assert_allclose(f[1], f[0], atol=1e-5 * np.abs(f[0]).max(), rtol=0)
+    np.testing.assert_allclose(v[1], v[0], atol=1e-6 * np.abs(v[0]).max(), rtol=0)
