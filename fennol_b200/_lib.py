@@ -100,6 +100,7 @@ _SIGNATURES = {
     "fennol_graph_build_noalloc": (I, [P, I, P, I, P, P, P, P, P, P, I, D, I, P, P, P, P, P, P]),
     "fennol_graph_noalloc_limits": (I, [P, P, P]),
     "fennol_graph_filter": (I, [P, I, P, P, P, P, P, I, D, I, P, P, P, P, P]),
+    "fennol_graph_filter_packed": (I, [P, I, P, P, P, P, P, I, D, I, P, P, P, P, P]),
     "fennol_aev_length": (I, [C.POINTER(AEVParams)]),
     "fennol_pack_atoms": (I, [P, P, I, P, P]),
     "fennol_aev_forward": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, I, P, P, I, P, P]),
@@ -108,7 +109,7 @@ _SIGNATURES = {
     "fennol_aev_backward_virial_staged": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, P, I, P, P, P, P, P]),
     "fennol_aev_stage_bytes": (SZ, [I, I]),
     "fennol_aev_forward_staged": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, I, P, P, I, P, SZ, P, P]),
-    "fennol_aev_forward_groups": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, I, P, P, I, P, I, P, SZ, P, P]),
+    "fennol_aev_forward_groups": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, I, P, P, I, P, I, P, SZ, P, P, P]),
     "fennol_aev_backward_staged": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, P, I, P, P, P, P]),
     "fennol_virial_reduce": (I, [P, I, P, I, D, P, P]),
     "fennol_aev_tangent": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, P, P, I, P, P]),

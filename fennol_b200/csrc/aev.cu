@@ -579,8 +579,8 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
               const float* __restrict__ sys_cell, const int* __restrict__ nbr_j,
               const unsigned* __restrict__ nbr_shift, const int* __restrict__ nbr_count, int cap,
               const AevConst K, const int* __restrict__ atom_row, int out_kind, void* __restrict__ out,
-              void* __restrict__ out_lo, int ld, int vec, const __grid_constant__ RowGroups rg, int* status,
-              char* __restrict__ stage_g) {
+              void* __restrict__ out_lo, int ld, int vec, const __grid_constant__ RowGroups rg,
+              float4* __restrict__ zero4, int* status, char* __restrict__ stage_g) {
   pdl_wait();
   extern __shared__ __align__(16) char smem_c[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -588,7 +588,9 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
   if (i >= n) return;
   const int S = K.S;
   Stage st = carve_stage(smem_c + (size_t)warp * stage_bytes(cap), cap);
+  if (zero4 && lane == 0) zero4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 pi = xyzs[i];
+  const int seen = status_peek(status, ST_ANG_MAXCOUNT);
   float c[9];
   load_cell(sys_cell, atom_sys[i], c);
   int cnt = nbr_count[i];
@@ -597,7 +599,7 @@ k_aev_forward(const float4* __restrict__ xyzs, int n, const int* __restrict__ at
   stage_row<true>(st, st.cntw, xyzs, pi, c, nbr_j, nbr_shift, (size_t)i * cap, cnt, K, lane, cnt_r, off_r, cnt_a,
                   off_a, na);
   if (lane == 0) {
-    status_max(status, ST_ANG_MAXCOUNT, na);
+    status_max(status, ST_ANG_MAXCOUNT, na, seen);
     if (na > st.capa) status_set(status, ST_ANG_OVERFLOW);
   }
   if (stage_g) {
@@ -1302,8 +1304,8 @@ extern "C" int fennol_pack_atoms(const float* coords, const int* species_idx, in
 static int aev_forward_launch(const float* xyzs, int natoms, const int* atom_sys, const float* sys_cell,
                               const int* nbr_j, const unsigned* nbr_shift, const int* nbr_count, int capacity,
                               const fennol_aev_params* p, const int* atom_row, int out_kind, void* out,
-                              void* out_lo, int ld, const unsigned long long* groups, int words, int* status,
-                              void* stage, void* stream) {
+                              void* out_lo, int ld, const unsigned long long* groups, int words, float* zero4,
+                              int* status, void* stage, void* stream) {
   AevConst K;
   if (!make_const(p, &K)) return FENNOL_ERR_UNSUPPORTED;
   if (natoms < 0 || capacity <= 0 || ld < K.F) return FENNOL_ERR_INVALID;
@@ -1326,7 +1328,7 @@ static int aev_forward_launch(const float* xyzs, int natoms, const int* atom_sys
     if (!smem) return false;
     if (launch_pdl(ks.fwd, blocks, kAevWarps * 32, smem, (cudaStream_t)stream, 
         (const float4*)xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, K,
-        atom_row, out_kind, out, out_lo, ld, vec, rg, status, (char*)stage) != cudaSuccess) return false;
+        atom_row, out_kind, out, out_lo, ld, vec, rg, (float4*)zero4, status, (char*)stage) != cudaSuccess) return false;
     return true;
   });
   if (!launched) return FENNOL_ERR_UNSUPPORTED;
@@ -1340,7 +1342,7 @@ extern "C" int fennol_aev_forward(const float* xyzs, int natoms, const int* atom
                                   const int* atom_row, int out_kind, void* out, void* out_lo, int ld,
                                   int* status, void* stream) {
   return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
-                            out_kind, out, out_lo, ld, nullptr, 0, status, nullptr, stream);
+                            out_kind, out, out_lo, ld, nullptr, 0, nullptr, status, nullptr, stream);
 }
 
 extern "C" size_t fennol_aev_stage_bytes(int natoms, int capacity) {
@@ -1356,7 +1358,7 @@ extern "C" int fennol_aev_forward_staged(const float* xyzs, int natoms, const in
   if (natoms > 0 && (!stage || ((uintptr_t)stage & 15) != 0)) return FENNOL_ERR_INVALID;
   if (stage_bytes_ < fennol_aev_stage_bytes(natoms, capacity)) return FENNOL_ERR_WORKSPACE;
   return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
-                            out_kind, out, out_lo, ld, nullptr, 0, status, stage, stream);
+                            out_kind, out, out_lo, ld, nullptr, 0, nullptr, status, stage, stream);
 }
 
 extern "C" int fennol_aev_forward_groups(const float* xyzs, int natoms, const int* atom_sys,
@@ -1364,12 +1366,12 @@ extern "C" int fennol_aev_forward_groups(const float* xyzs, int natoms, const in
                                          const int* nbr_count, int capacity, const fennol_aev_params* p,
                                          const int* atom_row, int out_kind, void* out, void* out_lo, int ld,
                                          const unsigned long long* host_groups, int group_words, void* stage,
-                                         size_t stage_bytes_, int* status, void* stream) {
+                                         size_t stage_bytes_, float* zero_forces4, int* status, void* stream) {
   if (host_groups && (long long)group_words * 64 * 16 < fennol_aev_length(p)) return FENNOL_ERR_INVALID;
-  if (stage && ((uintptr_t)stage & 15) != 0) return FENNOL_ERR_INVALID;
+  if ((((uintptr_t)stage | (uintptr_t)zero_forces4) & 15) != 0) return FENNOL_ERR_INVALID;
   if (stage && stage_bytes_ < fennol_aev_stage_bytes(natoms, capacity)) return FENNOL_ERR_WORKSPACE;
   return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
-                            out_kind, out, out_lo, ld, host_groups, group_words, status, stage, stream);
+                            out_kind, out, out_lo, ld, host_groups, group_words, zero_forces4, status, stage, stream);
 }
 
 static int aev_backward_launch(const float* xyzs, int natoms, const int* atom_sys, const float* sys_cell,

@@ -59,8 +59,16 @@ __device__ __forceinline__ float frac_exact(float vx, float vy, float vz, const 
   return __fadd_rn(__fadd_rn(__fmul_rn(vx, r[d]), __fmul_rn(vy, r[3 + d])), __fmul_rn(vz, r[6 + d]));
 }
 
-__device__ __forceinline__ void status_max(int* status, int word, int v) {
-  if (status) atomicMax(status + word, v);
+// Largest value of a status word.  Every row reports its length, and atomics on
+// one address take their turns (about 1 ns each: 98,304 rows 110 us, all of the
+// filter's time), so a row reports only what exceeds the word as the caller saw
+// it (status_peek, read early enough that nobody waits for it; an older value only
+// costs an atomic).
+__device__ __forceinline__ int status_peek(const int* status, int word) {
+  return status ? *(const volatile int*)(status + word) : 0;
+}
+__device__ __forceinline__ void status_max(int* status, int word, int v, int seen) {
+  if (status && v > seen) atomicMax(status + word, v);
 }
 __device__ __forceinline__ void status_set(int* status, int word) {
   if (status) atomicOr(status + word, 1);

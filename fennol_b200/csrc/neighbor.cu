@@ -215,13 +215,15 @@ __device__ __forceinline__ void row_append(bool keep, int j, unsigned sh, int* _
   count += __popc(m);
 }
 
+// seen: the row length that the status word held when the caller last looked
 __device__ __forceinline__ void row_finish(int i, int count, int cap, int* __restrict__ nbr_count, int* status,
-                                           int lane) {
+                                           int& seen, int lane) {
   if (lane == 0) {
     nbr_count[i] = count < cap ? count : cap;
     if (count > cap) status_set(status, ST_NBR_OVERFLOW);
-    status_max(status, ST_NBR_MAXCOUNT, count);
+    status_max(status, ST_NBR_MAXCOUNT, count, seen);
   }
+  seen = max(seen, count);
 }
 
 // ---------------------------------------------------------------------------
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(256) k_sort_cells(int c, GraphWs w, const int*
 __device__ __forceinline__ void cell_row(int i, const int* __restrict__ atom_sys, const SysView& sv,
                                          const GraphWs& w, float rc2, int cap, int* __restrict__ nbr_j,
                                          unsigned* __restrict__ nbr_shift, int* __restrict__ nbr_count,
-                                         int* status, int lane) {
+                                         int* status, int& seen, int lane) {
   const int cell = w.atom_cell[i];
   if (cell < 0) return;  // all-pairs system
   const int b = atom_sys[i];
@@ -347,7 +349,7 @@ __device__ __forceinline__ void cell_row(int i, const int* __restrict__ atom_sys
     }
     row_append(keep, j, sh, nbr_j, nbr_shift, base, cap, count, lane);
   }
-  row_finish(i, count, cap, nbr_count, status, lane);
+  row_finish(i, count, cap, nbr_count, status, seen, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -393,6 +395,7 @@ k_build_cells_staged(int ncells, const int* __restrict__ atom_sys, SysView sv, G
   // pre-test threshold: a little above rc^2, far beyond the rounding difference
   // between the pre-test's distance and the exact one
   const float rc_pre = sqrtf(rc2) + 0.05f, rc2_pre = rc_pre * rc_pre;
+  int seen = status_peek(status, ST_NBR_MAXCOUNT);
   for (int cell = blockIdx.x; cell < ncells; cell += gridDim.x) {
     const int a0 = w.starts[cell], na = w.starts[cell + 1] - a0;
     if (na == 0) continue;  // block-uniform
@@ -518,12 +521,12 @@ k_build_cells_staged(int ncells, const int* __restrict__ atom_sys, SysView sv, G
             row_append(keep, j, sh, nbr_j, nbr_shift, base, cap, count, lane);
           }
         }
-        row_finish(i, count, cap, nbr_count, status, lane);
+        row_finish(i, count, cap, nbr_count, status, seen, lane);
         __syncwarp();  // the queue is reused by the warp's next atom
       }
     } else {
       for (int a = warp; a < na; a += kCellWarps)
-        cell_row(w.cell_atoms[a0 + a], atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift, nbr_count, status, lane);
+        cell_row(w.cell_atoms[a0 + a], atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift, nbr_count, status, seen, lane);
     }
     __syncthreads();  // the stencil tables and candidates are reused by the next cell
   }
@@ -535,7 +538,7 @@ k_build_cells_staged(int ncells, const int* __restrict__ atom_sys, SysView sv, G
 __device__ __forceinline__ void allpairs_row(int i, const int* __restrict__ atom_sys, const SysView& sv,
                                              const GraphWs& w, float rc2, int cap, int* __restrict__ nbr_j,
                                              unsigned* __restrict__ nbr_shift, int* __restrict__ nbr_count,
-                                             int* status, int lane) {
+                                             int* status, int& seen, int lane) {
   if (w.atom_cell[i] >= 0) return;  // cell-list system
   const size_t base = (size_t)i * cap;
   int b = atom_sys[i];
@@ -564,7 +567,7 @@ __device__ __forceinline__ void allpairs_row(int i, const int* __restrict__ atom
           row_append(keep, j, sh, nbr_j, nbr_shift, base, cap, count, lane);
         }
       }
-  row_finish(i, count, cap, nbr_count, status, lane);
+  row_finish(i, count, cap, nbr_count, status, seen, lane);
 }
 
 // Also counts the rebuild (one per enabled build) in the status words.
@@ -576,15 +579,23 @@ k_build_allpairs(int n, const int* __restrict__ atom_sys, SysView sv, GraphWs w,
   if (enable_flag && *enable_flag == 0) return;
   if (status && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(status + ST_REBUILD_COUNT, 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int seen = status_peek(status, ST_NBR_MAXCOUNT);
   for (int i = blockIdx.x * kBuildWarps + warp; i < n; i += gridDim.x * kBuildWarps)
-    allpairs_row(i, atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift, nbr_count, status, lane);
+    allpairs_row(i, atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift, nbr_count, status, seen, lane);
 }
 
 
 // ---------------------------------------------------------------------------
-// Filter a list to a smaller cutoff (update_skin / GraphFilter).
+// Filter a list to a smaller cutoff (update_skin / GraphFilter).  Bound by the
+// gathers of the neighbour positions: a 32-byte line from L2 for each of the 100
+// entries of a skin row, 315 MB for 98,304 atoms of water (the lists themselves,
+// 125 MB, would take 20 us).  PACKED reads (x, y, z, species) rows with one load
+// where [n][3] rows take three.  110 us -> 65 without an atomic per row, 58 with
+// packed rows, 56 with entries that do not wait for the row's length and five
+// blocks per SM; 12,288 atoms 14.6 -> 10.9 us.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+template <bool PACKED>
+__global__ void __launch_bounds__(256, 5)
 k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_sys,
          const float* __restrict__ sys_cell, const int* __restrict__ in_j,
          const unsigned* __restrict__ in_shift, const int* __restrict__ in_count, int in_cap,
@@ -597,7 +608,12 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   int i = warp;
   int b = atom_sys[i];
   const float* c = sys_cell ? sys_cell + 9 * b : nullptr;
-  float xi = coords[3 * i], yi = coords[3 * i + 1], zi = coords[3 * i + 2];
+  auto position = [&](int k) {
+    if constexpr (PACKED) return __ldg(reinterpret_cast<const float4*>(coords) + k);
+    else return make_float4(coords[3 * k], coords[3 * k + 1], coords[3 * k + 2], 0.f);
+  };
+  const float4 pi = position(i);
+  const int seen = status_peek(status, ST_FILTER_MAXCOUNT);
   int cnt = in_count[i];
   if (cnt > in_cap) cnt = in_cap;
   size_t ib = (size_t)i * in_cap, ob = (size_t)i * out_cap;
@@ -606,30 +622,29 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   // position loads are in flight together, then the tests and the ordered
   // ballot compaction run round by round (same rows as one round at a time)
   constexpr int kFilterRounds = 4;
-  for (int k0 = 0; k0 < cnt; k0 += 32 * kFilterRounds) {
+  for (int k0 = 0; k0 == 0 || k0 < cnt; k0 += 32 * kFilterRounds) {
     int j[kFilterRounds];
     unsigned sh[kFilterRounds];
+    // entries of the row's capacity, not of its length: they do not wait for it
 #pragma unroll
     for (int u = 0; u < kFilterRounds; ++u) {
       const int k = k0 + 32 * u + lane;
-      j[u] = k < cnt ? in_j[ib + k] : -1;
-      sh[u] = k < cnt ? in_shift[ib + k] : 0u;
+      j[u] = k < in_cap ? in_j[ib + k] : -1;
+      sh[u] = k < in_cap ? in_shift[ib + k] : 0u;
     }
-    float px[kFilterRounds], py[kFilterRounds], pz[kFilterRounds];
 #pragma unroll
-    for (int u = 0; u < kFilterRounds; ++u) {
-      const int jj = j[u] < 0 ? i : j[u];
-      px[u] = coords[3 * jj];
-      py[u] = coords[3 * jj + 1];
-      pz[u] = coords[3 * jj + 2];
-    }
+    for (int u = 0; u < kFilterRounds; ++u)
+      if (k0 + 32 * u + lane >= cnt) j[u] = -1;
+    float4 p[kFilterRounds];
+#pragma unroll
+    for (int u = 0; u < kFilterRounds; ++u) p[u] = position(j[u] < 0 ? i : j[u]);
 #pragma unroll
     for (int u = 0; u < kFilterRounds; ++u) {
       bool keep = false;
       if (j[u] >= 0) {
-        float vx = __fsub_rn(px[u], xi);
-        float vy = __fsub_rn(py[u], yi);
-        float vz = __fsub_rn(pz[u], zi);
+        float vx = __fsub_rn(p[u].x, pi.x);
+        float vy = __fsub_rn(p[u].y, pi.y);
+        float vz = __fsub_rn(p[u].z, pi.z);
         if (sh[u] && c) {
           int sx, sy, sz;
           unpack_shift(sh[u], sx, sy, sz);
@@ -651,7 +666,7 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   if (lane == 0) {
     out_count[i] = count < out_cap ? count : out_cap;
     if (count > out_cap) status_set(status, ST_FILTER_OVERFLOW);
-    status_max(status, ST_FILTER_MAXCOUNT, count);
+    status_max(status, ST_FILTER_MAXCOUNT, count, seen);
   }
 }
 
@@ -751,7 +766,8 @@ extern "C" int fennol_graph_build(const float* coords, int natoms, const int* at
   return FENNOL_OK;
 }
 
-extern "C" int fennol_graph_filter(const float* coords, int natoms, const int* atom_sys,
+template <bool PACKED>
+static int filter_launch(const float* coords, int natoms, const int* atom_sys,
                                    const float* sys_cell, const int* in_j, const unsigned* in_shift,
                                    const int* in_count, int in_capacity, double cutoff,
                                    int out_capacity, int* out_j, unsigned* out_shift, int* out_count,
@@ -763,11 +779,30 @@ extern "C" int fennol_graph_filter(const float* coords, int natoms, const int* a
   float rc2 = (float)(cutoff * cutoff);
   int threads = 256;
   long long blocks = ((long long)natoms * 32 + threads - 1) / threads;
-  FNL_LAUNCH_PDL(k_filter, (unsigned)blocks, threads, 0, (cudaStream_t)stream, 
+  FNL_LAUNCH_PDL(k_filter<PACKED>, (unsigned)blocks, threads, 0, (cudaStream_t)stream, 
       coords, natoms, atom_sys, sys_cell, in_j, in_shift, in_count, in_capacity, rc2, out_capacity,
       out_j, out_shift, out_count, status);
   FNL_CHECK_LAUNCH();
   return FENNOL_OK;
+}
+
+extern "C" int fennol_graph_filter(const float* coords, int natoms, const int* atom_sys,
+                                   const float* sys_cell, const int* in_j, const unsigned* in_shift,
+                                   const int* in_count, int in_capacity, double cutoff,
+                                   int out_capacity, int* out_j, unsigned* out_shift, int* out_count,
+                                   int* status, void* stream) {
+  return filter_launch<false>(coords, natoms, atom_sys, sys_cell, in_j, in_shift, in_count, in_capacity, cutoff,
+                              out_capacity, out_j, out_shift, out_count, status, stream);
+}
+
+extern "C" int fennol_graph_filter_packed(const float* xyzs, int natoms, const int* atom_sys,
+                                          const float* sys_cell, const int* in_j, const unsigned* in_shift,
+                                          const int* in_count, int in_capacity, double cutoff,
+                                          int out_capacity, int* out_j, unsigned* out_shift, int* out_count,
+                                          int* status, void* stream) {
+  if (((uintptr_t)xyzs & 15) != 0) return FENNOL_ERR_INVALID;
+  return filter_launch<true>(xyzs, natoms, atom_sys, sys_cell, in_j, in_shift, in_count, in_capacity, cutoff,
+                             out_capacity, out_j, out_shift, out_count, status, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -196,7 +196,7 @@ class MDEngine:
             g.build(lay, self.coords, ws.status, st)
             if self.verify_stride:
                 self.x_ref.copy_(self.x)  # the stream is torch's current one (captured or not)
-        g.filter(lay, self.coords, ws.status, st)
+        g.filter(lay, ws.xyzs, ws.status, st)
         # the finite check runs once per chunk (run), not every step
         self.pot.launch_forces(lay, g, ws, st, True, check_finite=False)
 

@@ -337,9 +337,12 @@ class GraphBuffers:
              _ptr(enable_flag), stream)
 
     def filter(self, layout: BatchLayout, coords: torch.Tensor, status: torch.Tensor, stream: int):
+        """Radial rows from the skin rows; ``coords``: positions [N, 3], or the
+        packed rows [N, 4] of the same positions."""
         if self.skin <= 0:
             return
-        call("fennol_graph_filter", coords.data_ptr(), layout.n, layout.t_atom_sys.data_ptr(),
+        name = "fennol_graph_filter_packed" if coords.shape[1] == 4 else "fennol_graph_filter"
+        call(name, coords.data_ptr(), layout.n, layout.t_atom_sys.data_ptr(),
              layout.t_cell.data_ptr(), self.nbr_j.data_ptr(), self.nbr_s.data_ptr(), self.nbr_n.data_ptr(),
              self.cap, float(self.cutoff), self.cap_r, self.rad_j.data_ptr(), self.rad_s.data_ptr(),
              self.rad_n.data_ptr(), status.data_ptr(), stream)
@@ -539,7 +542,7 @@ class ANIPotential:
              layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
              g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.aev_kind, ws.x.data_ptr(), _ptr(ws.x_lo),
              ws.x.shape[1], groups.ctypes.data, groups.size, _ptr(stage), 0 if stage is None else stage.numel(),
-             ws.status.data_ptr(), stream)
+             ws.forces4.data_ptr() if want_forces else None, ws.status.data_ptr(), stream)
         call("fennol_mlp_energy_grad_groups", self.precision, layout.rows, layout.ntiles,
              layout.t_tile_species.data_ptr(), layout.t_tile_row.data_ptr(), C_ptr(self.mlp.struct),
              ws.x.data_ptr(), _ptr(ws.x_lo), groups.ctypes.data, groups.ctypes.data, groups.size,
@@ -552,8 +555,7 @@ class ANIPotential:
         call("fennol_energy_reduce", ws.e_rows.data_ptr(), layout.t_atom_row.data_ptr(), n,
              layout.t_sys_start.data_ptr(), layout.nsys, float(self.unit_scale), ws.energy.data_ptr(),
              ws.e_atom.data_ptr(), ws.energy_ws.data_ptr(), ws.energy_ws.numel(), stream)
-        if want_forces and want_virial:
-            ws.forces4.zero_()
+        if want_forces and want_virial:  # forces4 was cleared by the forward
             av, vir = ws.virial_buffers(layout)
             args = (ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(), layout.t_cell.data_ptr(),
                     g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(), g.cap_r, lib_p,
@@ -566,13 +568,11 @@ class ANIPotential:
             call("fennol_virial_reduce", av.data_ptr(), n, layout.t_sys_start.data_ptr(), layout.nsys,
                  float(self.unit_scale), vir.data_ptr(), stream)
         elif stage is not None:
-            ws.forces4.zero_()
             call("fennol_aev_backward_staged", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
                  layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
                  g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1],
                  ws.forces4.data_ptr(), stage.data_ptr(), ws.status.data_ptr(), stream)
         elif want_forces:
-            ws.forces4.zero_()
             call("fennol_aev_backward", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
                  layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
                  g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1],

@@ -294,7 +294,7 @@ class _MDLane:
              ws.xyzs.data_ptr(), st["x_ref"].data_ptr(), 0.5 * e.skin, st["flag"].data_ptr(), s)
         launch_flagged_rebuild(g, lay, st["coords"], ws.status, st["flag"], st["x"], st["x_ref"], s,
                                self.body_stream.cuda_stream)
-        g.filter(lay, st["coords"], ws.status, s)
+        g.filter(lay, ws.xyzs, ws.status, s)
         pot.launch_forces(lay, g, ws, s, True)
 
     # ------------------------------------------------------------ segments

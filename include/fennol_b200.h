@@ -156,6 +156,13 @@ int fennol_graph_filter(const float* coords, int natoms, const int* atom_sys,
                         int* out_j, unsigned* out_shift, int* out_count, int* status,
                         void* stream);
 
+/* The same from the packed rows of fennol_pack_atoms (x, y, z, species; 16-byte aligned). */
+int fennol_graph_filter_packed(const float* xyzs, int natoms, const int* atom_sys,
+                        const float* sys_cell, const int* in_j, const unsigned* in_shift,
+                        const int* in_count, int in_capacity, double cutoff, int out_capacity,
+                        int* out_j, unsigned* out_shift, int* out_count, int* status,
+                        void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* ANI atomic environment vectors                                            */
 /* ------------------------------------------------------------------------ */
@@ -274,14 +281,15 @@ int fennol_aev_backward_staged(const float* xyzs, int natoms, const int* atom_sy
  * other columns of out and out_lo stay as they are.  The caller names every
  * group that can be non-zero (fennol_aev_active_groups for a species set);
  * the features of a block outside them are stored all the same.  stage: NULL,
- * or as for fennol_aev_forward_staged.
+ * or as for fennol_aev_forward_staged.  zero_forces4: NULL, or the forces4 of the
+ * adjoint that follows (natoms x 4, 16-byte aligned), which this call clears.
  */
 int fennol_aev_forward_groups(const float* xyzs, int natoms, const int* atom_sys,
                               const float* sys_cell, const int* nbr_j, const unsigned* nbr_shift,
                               const int* nbr_count, int capacity, const fennol_aev_params* p,
                               const int* atom_row, int out_kind, void* out, void* out_lo, int ld,
                               const unsigned long long* host_groups, int group_words, void* stage,
-                              size_t stage_bytes, int* status, void* stream);
+                              size_t stage_bytes, float* zero_forces4, int* status, void* stream);
 
 /*
  * fennol_aev_backward that also writes, per centre atom i, the 3x3 sum over

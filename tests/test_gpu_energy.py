@@ -200,8 +200,10 @@ def test_forward_groups_and_staged_virial(cuda_device, precision, off):
         if words is None:
             call("fennol_aev_forward", *args, *out, ws.status.data_ptr(), st)
         else:
+            ws.forces4.fill_(3.0)
             call("fennol_aev_forward_groups", *args, *out, words.ctypes.data, words.size, g.aev_stage.data_ptr(),
-                 g.aev_stage.numel(), ws.status.data_ptr(), st)
+                 g.aev_stage.numel(), ws.forces4.data_ptr(), ws.status.data_ptr(), st)
+            assert int(torch.count_nonzero(ws.forces4[:lay.n])) == 0
         got.append([b[off:].view(rows, d0)[lay.t_atom_row.long(), :F].float().cpu().numpy() for b in bufs])
     for k, (full, part) in enumerate(zip(*got)):
         np.testing.assert_array_equal(part[:, named], full[:, named])

@@ -247,3 +247,35 @@ def test_aev_on_reference_graphs(cuda_device, name):
     r = ani_ref.energy_and_forces(d["coordinates"], d["species"], nat, p.weights, AEVConfig(), MLPConfig(),
                                   cells=cells, minimum_image=mi, need_forces=False, return_aev=True)
     np.testing.assert_allclose(got, r["aev"], rtol=1e-4, atol=2e-5)
+
+
+@pytest.mark.parametrize("n_side,skin,cap", [(8, 1.0, 150), (8, 2.5, 233), (10, 0.3, 97), (0, 1.0, 61)])
+def test_packed_filter_matches_plain(pot, cuda_device, n_side, skin, cap):
+    """The filter gives the same rows from packed positions as from [N, 3] ones
+    (row capacities off the 32-entry rounds, rows longer than the 128 entries in
+    flight, molecules without a cell), and the status words hold the longest row."""
+    if n_side:
+        s = water_box(n_side, seed=20)
+        xyz, sp, nat, cells = s.coordinates, s.species, [s.natoms], s.cell[None]
+    else:
+        mols = molecule_batch(7, seed=21)
+        xyz, sp = np.concatenate([m.coordinates for m in mols]), np.concatenate([m.species for m in mols])
+        nat, cells = [m.natoms for m in mols], None
+    lay = pot.layout(sp, nat, cells)
+    coords = torch.tensor(xyz, dtype=torch.float32, device=cuda_device)
+    packed = torch.cat([coords, torch.zeros_like(coords[:, :1])], 1).contiguous()
+    status = torch.zeros(_lib.STATUS_WORDS, dtype=torch.int32, device=cuda_device)
+    g = GraphBuffers(lay, 5.2, skin, cap, 128)
+    st = torch.cuda.current_stream().cuda_stream
+    g.build(lay, coords, status, st)
+    rows = []
+    for pos in (coords, packed):
+        g.rad_j.zero_(), g.rad_s.zero_(), g.rad_n.zero_()
+        g.filter(lay, pos, status, st)
+        rows.append([t.cpu().numpy().copy() for t in (g.rad_j, g.rad_s, g.rad_n)])
+    for a, b in zip(*rows):
+        np.testing.assert_array_equal(a, b)
+    words = status.cpu().numpy()
+    assert words[_lib.ST_NBR_OVERFLOW] == 0 and words[_lib.ST_FILTER_OVERFLOW] == 0
+    assert words[_lib.ST_NBR_MAXCOUNT] == int(g.nbr_n.max()) > 0
+    assert words[_lib.ST_FILTER_MAXCOUNT] == rows[0][2].max() > 0
