@@ -121,6 +121,7 @@ _SIGNATURES = {
     "fennol_aev_active_chunks": (ULL, [C.POINTER(AEVParams), C.c_uint]),
     "fennol_energy_workspace_bytes": (SZ, [I, I]),
     "fennol_energy_reduce": (I, [P, P, I, P, I, D, P, P, P, SZ, P]),
+    "fennol_energy_reduce_behind_adjoint": (I, [P, P, I, P, I, D, P, P, P, SZ, P]),
     "fennol_forces_finalize": (I, [P, I, F, P, P]),
     "fennol_md_step": (I, [I, D, P, P, P, P, D, D, P, ULL, P, P, P, P, P, D, P, P]),
     "fennol_md_step_systems": (I, [I, I, D, P, P, P, P, D, D, P, P, P, P, P, P, P, P, P, D, P, P]),

@@ -766,6 +766,7 @@ k_aev_backward(const float4* __restrict__ xyzs, int n, const int* __restrict__ a
                int ld, float4* __restrict__ forces, float* __restrict__ atom_virial, int* status,
                const char* __restrict__ stage_g) {
   pdl_wait();
+  pdl_trigger();  // the energy sum behind this kernel fills its tail
   extern __shared__ __align__(16) char smem_c[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * kAevWarps + warp;

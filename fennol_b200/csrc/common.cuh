@@ -92,6 +92,11 @@ __host__ __device__ __forceinline__ int triu_pair(int s1, int s2, int S) {
 // completed and its writes are visible (a no-op for ordinary launches).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Lets the next kernel of the stream start once every block of this one has come
+// here (its pdl_wait still returns only when this kernel is complete).  After
+// this kernel's own pdl_wait, so that what came before it is complete by then.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args&&... args) {

@@ -31,13 +31,21 @@ __device__ __forceinline__ int red_chunks(const int* sys_start, int b) {
   return max(1, (sys_start[b + 1] - sys_start[b] + kRedChunk - 1) / kRedChunk);
 }
 
+// A chain of dependent loads (row numbers, rows, partials), nothing else: the four
+// values of a thread and the partials of a system are in flight together, and with
+// `behind` the kernel runs while the one before it in the stream drains (it
+// reads nothing of that kernel and waits for it at its end, so that whatever
+// follows still comes after both).  12,288 / 98,304 atoms alone: 9.5 / 12.8 us ->
+// 6.3 / 7.5 us; behind the adjoint 8 us of a 12,288-atom MD step of 193.
 __global__ void __launch_bounds__(256) k_energy_sum(const float* __restrict__ e_rows, const int* __restrict__ atom_row,
                                                    const int* __restrict__ sys_start, int nsys, int nslots, double scale,
                                                    double* __restrict__ partial, double* __restrict__ e_atom,
-                                                   double* __restrict__ energy, unsigned* __restrict__ ticket) {
-  pdl_wait();
+                                                   double* __restrict__ energy, unsigned* __restrict__ ticket,
+                                                   bool behind) {
+  if (!behind) pdl_wait();
   __shared__ double part[256];
   __shared__ bool last;
+  const int tid = threadIdx.x, lane = tid & 31;
   for (int w = blockIdx.x; w < nslots; w += gridDim.x) {
     // the system b with base(b) <= w < base(b + 1)
     int lo = 0, hi = nsys - 1;
@@ -47,36 +55,61 @@ __global__ void __launch_bounds__(256) k_energy_sum(const float* __restrict__ e_
     }
     const int b = lo, c = w - red_base(sys_start, b);
     if (c < 0 || c >= red_chunks(sys_start, b)) continue;  // a gap slot (uniform per block)
-    const int i0 = sys_start[b] + c * kRedChunk;
-    const int i1 = min(i0 + kRedChunk, sys_start[b + 1]);
+    const int i0 = sys_start[b] + c * kRedChunk + tid;
+    const int i1 = min(i0 - tid + kRedChunk, sys_start[b + 1]);
     double s = 0.0;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-      double e = scale * (double)e_rows[atom_row[i]];
-      if (e_atom) e_atom[i] = e;
-      s += e;
-    }
-    part[threadIdx.x] = s;
+    int row[kRedChunk / 256];
+    float v[kRedChunk / 256];
+#pragma unroll
+    for (int k = 0; k < kRedChunk / 256; ++k) row[k] = i0 + 256 * k < i1 ? atom_row[i0 + 256 * k] : -1;
+#pragma unroll
+    for (int k = 0; k < kRedChunk / 256; ++k) v[k] = row[k] >= 0 ? __ldcg(e_rows + row[k]) : 0.f;
+#pragma unroll
+    for (int k = 0; k < kRedChunk / 256; ++k)
+      if (row[k] >= 0) {
+        const double e = scale * (double)v[k];
+        if (e_atom) e_atom[i0 + 256 * k] = e;
+        s += e;
+      }
+    part[tid] = s;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
+    for (int o = 128; o >= 32; o >>= 1) {
+      if (tid < o) part[tid] += part[tid + o];
       __syncthreads();
     }
-    if (threadIdx.x == 0) partial[w] = part[0];
+    if (tid < 32) {
+      s = part[tid];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (tid == 0) partial[w] = s;
+    }
     __syncthreads();
   }
   // the last block to arrive sums the partials (all written before its ticket)
   __threadfence();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  if (tid == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int b = threadIdx.x; b < nsys; b += blockDim.x) {
-    const int base = red_base(sys_start, b), nc = red_chunks(sys_start, b);
-    double s = 0.0;
-    for (int k = 0; k < nc; ++k) s += __ldcg(partial + base + k);
-    energy[b] = s;
+  if (last) {
+    __threadfence();
+    if (nsys > 8) {  // thread per system
+      for (int b = tid; b < nsys; b += blockDim.x) {
+        const int base = red_base(sys_start, b), nc = red_chunks(sys_start, b);
+        double s = 0.0;
+        for (int k = 0; k < nc; ++k) s += __ldcg(partial + base + k);
+        energy[b] = s;
+      }
+    } else if (tid >> 5 < nsys) {  // warp per system, 32 partials at a time, added in their order
+      const int b = tid >> 5, base = red_base(sys_start, b), nc = red_chunks(sys_start, b);
+      double s = 0.0;
+      for (int k0 = 0; k0 < nc; k0 += 32) {
+        const double p = k0 + lane < nc ? __ldcg(partial + base + k0 + lane) : 0.0;
+        for (int k = 0; k < min(nc - k0, 32); ++k) s += __shfl_sync(0xffffffffu, p, k);
+      }
+      if (lane == 0) energy[b] = s;
+    }
+    if (tid == 0) *ticket = 0u;  // ready for the next call
   }
-  if (threadIdx.x == 0) *ticket = 0u;  // ready for the next call
+  if (behind) pdl_wait();
 }
 
 __global__ void k_forces_finalize(const float4* __restrict__ f4, int n, float scale, float* __restrict__ f) {
@@ -289,10 +322,9 @@ extern "C" int fennol_virial_reduce(const float* atom_virial, int natoms, const 
   return FENNOL_OK;
 }
 
-extern "C" int fennol_energy_reduce(const float* e_rows, const int* atom_row, int natoms,
-                                    const int* sys_start, int nsys, double scale, double* energy,
-                                    double* e_atom, void* workspace, size_t workspace_bytes,
-                                    void* stream) {
+static int energy_reduce(const float* e_rows, const int* atom_row, int natoms, const int* sys_start, int nsys,
+                         double scale, double* energy, double* e_atom, void* workspace, size_t workspace_bytes,
+                         bool behind, void* stream) {
   if (natoms < 0 || nsys < 0) return FENNOL_ERR_INVALID;
   if (nsys == 0) return FENNOL_OK;
   if (!sys_start || !energy || !workspace || (natoms > 0 && (!e_rows || !atom_row))) return FENNOL_ERR_INVALID;
@@ -304,9 +336,25 @@ extern "C" int fennol_energy_reduce(const float* e_rows, const int* atom_row, in
   const int nslots = natoms / kRedChunk + nsys + 1;
   const int blocks = nslots < 4 * 148 ? nslots : 4 * 148;
   FNL_LAUNCH_PDL(k_energy_sum, blocks, 256, 0, st, e_rows, atom_row, sys_start, nsys, nslots, scale, partial, e_atom,
-                 energy, ticket);
+                 energy, ticket, behind);
   FNL_CHECK_LAUNCH();
   return FENNOL_OK;
+}
+
+extern "C" int fennol_energy_reduce(const float* e_rows, const int* atom_row, int natoms,
+                                    const int* sys_start, int nsys, double scale, double* energy,
+                                    double* e_atom, void* workspace, size_t workspace_bytes,
+                                    void* stream) {
+  return energy_reduce(e_rows, atom_row, natoms, sys_start, nsys, scale, energy, e_atom, workspace, workspace_bytes,
+                       false, stream);
+}
+
+extern "C" int fennol_energy_reduce_behind_adjoint(const float* e_rows, const int* atom_row, int natoms,
+                                                   const int* sys_start, int nsys, double scale, double* energy,
+                                                   double* e_atom, void* workspace, size_t workspace_bytes,
+                                                   void* stream) {
+  return energy_reduce(e_rows, atom_row, natoms, sys_start, nsys, scale, energy, e_atom, workspace, workspace_bytes,
+                       natoms > 0, stream);
 }
 
 extern "C" int fennol_forces_finalize(const float* forces4, int natoms, float scale, float* forces,

@@ -524,7 +524,7 @@ class ANIPotential:
     def launch_forces(self, layout: BatchLayout, g: GraphBuffers, ws: Workspace, stream: int,
                       want_forces: bool = True, want_virial: bool = False,
                       ghost_rows: Optional[torch.Tensor] = None, check_finite: bool = True):
-        """AEV -> MLP -> energies (and adjoint -> forces) from the current radial
+        """AEV -> MLP (-> adjoint -> forces) -> energies from the current radial
         list.  ``ghost_rows``: MLP rows of centres whose energy does not count
         (their row energy and dE/dAEV are cleared before the sum and the adjoint).
         ``check_finite``: one more launch sets status[ST_NONFINITE] when the
@@ -552,31 +552,26 @@ class ANIPotential:
             ws.e_rows.index_fill_(0, ghost_rows, 0.0)
             if want_forces:
                 ws.dx.index_fill_(0, ghost_rows, 0.0)
-        call("fennol_energy_reduce", ws.e_rows.data_ptr(), layout.t_atom_row.data_ptr(), n,
-             layout.t_sys_start.data_ptr(), layout.nsys, float(self.unit_scale), ws.energy.data_ptr(),
-             ws.e_atom.data_ptr(), ws.energy_ws.data_ptr(), ws.energy_ws.numel(), stream)
-        if want_forces and want_virial:  # forces4 was cleared by the forward
-            av, vir = ws.virial_buffers(layout)
+        sums = (ws.e_rows.data_ptr(), layout.t_atom_row.data_ptr(), n, layout.t_sys_start.data_ptr(), layout.nsys,
+                float(self.unit_scale), ws.energy.data_ptr(), ws.e_atom.data_ptr(), ws.energy_ws.data_ptr(),
+                ws.energy_ws.numel(), stream)
+        if want_forces:  # forces4 was cleared by the forward
+            name = "fennol_aev_backward"
             args = (ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(), layout.t_cell.data_ptr(),
                     g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(), g.cap_r, lib_p,
-                    layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1], ws.forces4.data_ptr(),
-                    av.data_ptr())
+                    layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1], ws.forces4.data_ptr())
+            if want_virial:
+                av, vir = ws.virial_buffers(layout)
+                name, args = name + "_virial", args + (av.data_ptr(),)
             if stage is not None:
-                call("fennol_aev_backward_virial_staged", *args, stage.data_ptr(), ws.status.data_ptr(), stream)
-            else:
-                call("fennol_aev_backward_virial", *args, ws.status.data_ptr(), stream)
-            call("fennol_virial_reduce", av.data_ptr(), n, layout.t_sys_start.data_ptr(), layout.nsys,
-                 float(self.unit_scale), vir.data_ptr(), stream)
-        elif stage is not None:
-            call("fennol_aev_backward_staged", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
-                 layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
-                 g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1],
-                 ws.forces4.data_ptr(), stage.data_ptr(), ws.status.data_ptr(), stream)
-        elif want_forces:
-            call("fennol_aev_backward", ws.xyzs.data_ptr(), n, layout.t_atom_sys.data_ptr(),
-                 layout.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(),
-                 g.cap_r, lib_p, layout.t_atom_row.data_ptr(), ws.dx.data_ptr(), ws.dx.shape[1],
-                 ws.forces4.data_ptr(), ws.status.data_ptr(), stream)
+                name, args = name + "_staged", args + (stage.data_ptr(),)
+            call(name, *args, ws.status.data_ptr(), stream)
+            call("fennol_energy_reduce_behind_adjoint", *sums)
+            if want_virial:
+                call("fennol_virial_reduce", av.data_ptr(), n, layout.t_sys_start.data_ptr(), layout.nsys,
+                     float(self.unit_scale), vir.data_ptr(), stream)
+        else:
+            call("fennol_energy_reduce", *sums)
         if check_finite:
             _lib.check_finite([ws.xyzs[:n], ws.energy, ws.forces4[:n] if want_forces else None], ws.status,
                               stream)

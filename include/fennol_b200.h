@@ -538,6 +538,16 @@ int fennol_energy_reduce(const float* e_rows, const int* atom_row, int natoms,
                          const int* sys_start, int nsys, double scale, double* energy,
                          double* e_atom, void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * The same for a call directly behind fennol_aev_backward (any form) on the same
+ * stream: it may run while that kernel drains.  e_rows must have been complete
+ * before the adjoint was enqueued, and the adjoint must have had atoms > 0
+ * exactly when this call has.
+ */
+int fennol_energy_reduce_behind_adjoint(const float* e_rows, const int* atom_row, int natoms,
+                         const int* sys_start, int nsys, double scale, double* energy,
+                         double* e_atom, void* workspace, size_t workspace_bytes, void* stream);
+
 /* forces[i*3+k] = scale * forces4[i*4+k] (float32 output). */
 int fennol_forces_finalize(const float* forces4, int natoms, float scale, float* forces,
                            void* stream);
