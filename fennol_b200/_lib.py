@@ -109,6 +109,7 @@ _SIGNATURES = {
     "fennol_aev_backward_virial_staged": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, P, I, P, P, P, P, P]),
     "fennol_aev_stage_bytes": (SZ, [I, I]),
     "fennol_aev_forward_staged": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, I, P, P, I, P, SZ, P, P]),
+    "fennol_aev_gather_rows": (I, [P, P, I, I, P, I, I, P, P]),
     "fennol_aev_forward_groups": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, I, P, P, I, P, I, P, SZ, P, P, P]),
     "fennol_aev_backward_staged": (I, [P, I, P, P, P, P, P, I, C.POINTER(AEVParams), P, P, I, P, P, P, P]),
     "fennol_virial_reduce": (I, [P, I, P, I, D, P, P]),

@@ -1204,6 +1204,54 @@ __global__ void k_pack(const float* __restrict__ coords, const int* __restrict__
   xyzs[i] = make_float4(coords[3 * i], coords[3 * i + 1], coords[3 * i + 2], __int_as_float(sp[i]));
 }
 
+// Rows in atom order as float32 (hi + lo): out[i][0..width) = row atom_row[i].  A
+// block per atom, four columns per thread (vec: 16-byte aligned rows, width and ld
+// multiples of 4); bound by memory traffic (8 bytes a value).  6,503 rows of 1008
+// FP16 hi + lo columns: 14 us, where conversions, gathers and a sum took 70.
+__global__ void __launch_bounds__(256) k_gather_rows(const void* __restrict__ x, const void* __restrict__ x_lo,
+                                                     int kind, int ld, const int* __restrict__ atom_row, int width,
+                                                     int vec, float* __restrict__ out) {
+  pdl_wait();
+  const size_t from = (size_t)atom_row[blockIdx.x] * ld, to = (size_t)blockIdx.x * width;
+  const bool lo = kind == FENNOL_AEV_BF16X2 || kind == FENNOL_AEV_F16X2;
+  auto half2_at = [&](unsigned w) {
+    if (kind == FENNOL_AEV_F16X2) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+  };
+  if (vec) {
+    for (int c = 4 * threadIdx.x; c < width; c += 1024) {
+      float4 v;
+      if (kind == FENNOL_AEV_F32) {
+        v = __ldg(reinterpret_cast<const float4*>((const float*)x + from + c));
+      } else {
+        const uint2 h = __ldg(reinterpret_cast<const uint2*>((const unsigned short*)x + from + c));
+        float2 a = half2_at(h.x), b = half2_at(h.y);
+        if (lo) {
+          const uint2 l = __ldg(reinterpret_cast<const uint2*>((const unsigned short*)x_lo + from + c));
+          const float2 al = half2_at(l.x), bl = half2_at(l.y);
+          a.x += al.x;
+          a.y += al.y;
+          b.x += bl.x;
+          b.y += bl.y;
+        }
+        v = make_float4(a.x, a.y, b.x, b.y);
+      }
+      *reinterpret_cast<float4*>(out + to + c) = v;
+    }
+  } else {
+    for (int c = threadIdx.x; c < width; c += 256) {
+      float v;
+      if (kind == FENNOL_AEV_F32) {
+        v = ((const float*)x)[from + c];
+      } else {
+        v = half2_at(((const unsigned short*)x)[from + c]).x;
+        if (lo) v += half2_at(((const unsigned short*)x_lo)[from + c]).x;
+      }
+      out[to + c] = v;
+    }
+  }
+}
+
 template <int RD, int AD, int AS, int ZN>
 struct AevKernels {
   static constexpr auto fwd = k_aev_forward<RD, AD, AS, ZN>;
@@ -1344,6 +1392,19 @@ extern "C" int fennol_aev_forward(const float* xyzs, int natoms, const int* atom
                                   int* status, void* stream) {
   return aev_forward_launch(xyzs, natoms, atom_sys, sys_cell, nbr_j, nbr_shift, nbr_count, capacity, p, atom_row,
                             out_kind, out, out_lo, ld, nullptr, 0, nullptr, status, nullptr, stream);
+}
+
+extern "C" int fennol_aev_gather_rows(const void* x, const void* x_lo, int out_kind, int ld, const int* atom_row,
+                                      int natoms, int width, float* out, void* stream) {
+  const bool lo = out_kind == FENNOL_AEV_BF16X2 || out_kind == FENNOL_AEV_F16X2;
+  if (natoms < 0 || width < 0 || ld < width || (!lo && out_kind != FENNOL_AEV_F32 && out_kind != FENNOL_AEV_BF16))
+    return FENNOL_ERR_INVALID;
+  if (natoms == 0 || width == 0) return FENNOL_OK;
+  if (!x || (lo && !x_lo) || !atom_row || !out) return FENNOL_ERR_INVALID;
+  const int vec = (((uintptr_t)x | (uintptr_t)(lo ? x_lo : x) | (uintptr_t)out) & 15) == 0 && ((ld | width) & 3) == 0;
+  FNL_LAUNCH_PDL(k_gather_rows, natoms, 256, 0, (cudaStream_t)stream, x, x_lo, out_kind, ld, atom_row, width, vec, out);
+  FNL_CHECK_LAUNCH();
+  return FENNOL_OK;
 }
 
 extern "C" size_t fennol_aev_stage_bytes(int natoms, int capacity) {

@@ -63,7 +63,7 @@ __device__ __forceinline__ float frac_exact(float vx, float vy, float vz, const 
 // one address take their turns (about 1 ns each: 98,304 rows 110 us, all of the
 // filter's time), so a row reports only what exceeds the word as the caller saw
 // it (status_peek, read early enough that nobody waits for it; an older value only
-// costs an atomic).
+// costs an atomic), and the list kernels report once per block.
 __device__ __forceinline__ int status_peek(const int* status, int word) {
   return status ? *(const volatile int*)(status + word) : 0;
 }

@@ -215,15 +215,24 @@ __device__ __forceinline__ void row_append(bool keep, int j, unsigned sh, int* _
   count += __popc(m);
 }
 
-// seen: the row length that the status word held when the caller last looked
+// longest: the longest row of this warp so far (report_longest)
 __device__ __forceinline__ void row_finish(int i, int count, int cap, int* __restrict__ nbr_count, int* status,
-                                           int& seen, int lane) {
+                                           int& longest, int lane) {
   if (lane == 0) {
     nbr_count[i] = count < cap ? count : cap;
     if (count > cap) status_set(status, ST_NBR_OVERFLOW);
-    status_max(status, ST_NBR_MAXCOUNT, count, seen);
   }
-  seen = max(seen, count);
+  longest = max(longest, count);
+}
+
+// Block-collective: the longest row of the block's warps, one atomic for all.
+__device__ __forceinline__ void report_longest(int* status, int word, int longest, int seen) {
+  __shared__ int block_longest;
+  if (threadIdx.x == 0) block_longest = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(&block_longest, longest);
+  __syncthreads();
+  if (threadIdx.x == 0) status_max(status, word, block_longest, seen);
 }
 
 // ---------------------------------------------------------------------------
@@ -289,7 +298,7 @@ __global__ void __launch_bounds__(256) k_sort_cells(int c, GraphWs w, const int*
 __device__ __forceinline__ void cell_row(int i, const int* __restrict__ atom_sys, const SysView& sv,
                                          const GraphWs& w, float rc2, int cap, int* __restrict__ nbr_j,
                                          unsigned* __restrict__ nbr_shift, int* __restrict__ nbr_count,
-                                         int* status, int& seen, int lane) {
+                                         int* status, int& longest, int lane) {
   const int cell = w.atom_cell[i];
   if (cell < 0) return;  // all-pairs system
   const int b = atom_sys[i];
@@ -349,7 +358,7 @@ __device__ __forceinline__ void cell_row(int i, const int* __restrict__ atom_sys
     }
     row_append(keep, j, sh, nbr_j, nbr_shift, base, cap, count, lane);
   }
-  row_finish(i, count, cap, nbr_count, status, seen, lane);
+  row_finish(i, count, cap, nbr_count, status, longest, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -401,7 +410,8 @@ k_build_cells_staged(int ncells, const int* __restrict__ atom_sys, SysView sv, G
   // pre-test threshold: a little above rc^2, far beyond the rounding difference
   // between the pre-test's distance and the exact one
   const float rc_pre = sqrtf(rc2) + 0.05f, rc2_pre = rc_pre * rc_pre;
-  int seen = status_peek(status, ST_NBR_MAXCOUNT);
+  const int seen = status_peek(status, ST_NBR_MAXCOUNT);
+  int longest = 0;
   for (int cell = blockIdx.x; cell < ncells; cell += gridDim.x) {
     const int a0 = w.starts[cell], na = w.starts[cell + 1] - a0;
     if (na == 0) continue;  // block-uniform
@@ -529,15 +539,16 @@ k_build_cells_staged(int ncells, const int* __restrict__ atom_sys, SysView sv, G
             row_append(keep, j, sh, nbr_j, nbr_shift, base, cap, count, lane);
           }
         }
-        row_finish(i, count, cap, nbr_count, status, seen, lane);
+        row_finish(i, count, cap, nbr_count, status, longest, lane);
         __syncwarp();  // the queue is reused by the warp's next atom
       }
     } else {
       for (int a = warp; a < na; a += kCellWarps)
-        cell_row(w.cell_atoms[a0 + a], atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift, nbr_count, status, seen, lane);
+        cell_row(w.cell_atoms[a0 + a], atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift, nbr_count, status, longest, lane);
     }
     __syncthreads();  // the stencil tables and candidates are reused by the next cell
   }
+  report_longest(status, ST_NBR_MAXCOUNT, longest, seen);
 }
 
 // ---------------------------------------------------------------------------
@@ -546,7 +557,7 @@ k_build_cells_staged(int ncells, const int* __restrict__ atom_sys, SysView sv, G
 __device__ __forceinline__ void allpairs_row(int i, const int* __restrict__ atom_sys, const SysView& sv,
                                              const GraphWs& w, float rc2, int cap, int* __restrict__ nbr_j,
                                              unsigned* __restrict__ nbr_shift, int* __restrict__ nbr_count,
-                                             int* status, int& seen, int lane) {
+                                             int* status, int& longest, int lane) {
   const size_t base = (size_t)i * cap;
   int b = atom_sys[i];
   int mode = sv.mode[b];
@@ -574,7 +585,7 @@ __device__ __forceinline__ void allpairs_row(int i, const int* __restrict__ atom
           row_append(keep, j, sh, nbr_j, nbr_shift, base, cap, count, lane);
         }
       }
-  row_finish(i, count, cap, nbr_count, status, seen, lane);
+  row_finish(i, count, cap, nbr_count, status, longest, lane);
 }
 
 // Also counts the rebuild (one per enabled build) in the status words.
@@ -586,7 +597,8 @@ k_build_allpairs(int n, const int* __restrict__ atom_sys, SysView sv, GraphWs w,
   if (enable_flag && *enable_flag == 0) return;
   if (status && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(status + ST_REBUILD_COUNT, 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int seen = status_peek(status, ST_NBR_MAXCOUNT);
+  const int seen = status_peek(status, ST_NBR_MAXCOUNT);
+  int longest = 0;
   // the warp's next 32 rows are looked up at once: those of cell-list systems are
   // not its business (98,304 atoms, none of them: 13.2 us row by row, 5.5 so)
   const int stride = gridDim.x * kBuildWarps;
@@ -595,8 +607,9 @@ k_build_allpairs(int n, const int* __restrict__ atom_sys, SysView sv, GraphWs w,
     unsigned mine = __ballot_sync(0xffffffffu, i < n && w.atom_cell[i] < 0);
     for (; mine; mine &= mine - 1)
       allpairs_row((int)(i0 + (long long)(__ffs(mine) - 1) * stride), atom_sys, sv, w, rc2, cap, nbr_j, nbr_shift,
-                   nbr_count, status, seen, lane);
+                   nbr_count, status, longest, lane);
   }
+  report_longest(status, ST_NBR_MAXCOUNT, longest, seen);
 }
 
 
@@ -619,8 +632,7 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   pdl_wait();
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
-  if (warp >= n) return;
-  int i = warp;
+  const int i = min(warp, n - 1);  // the warps past the last row do it once more
   int b = atom_sys[i];
   const float* c = sys_cell ? sys_cell + 9 * b : nullptr;
   auto position = [&](int k) {
@@ -681,8 +693,8 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   if (lane == 0) {
     out_count[i] = count < out_cap ? count : out_cap;
     if (count > out_cap) status_set(status, ST_FILTER_OVERFLOW);
-    status_max(status, ST_FILTER_MAXCOUNT, count, seen);
   }
+  report_longest(status, ST_FILTER_MAXCOUNT, count, seen);
 }
 
 }  // namespace

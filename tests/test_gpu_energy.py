@@ -222,3 +222,58 @@ def test_forward_groups_and_staged_virial(cuda_device, precision, off):
     assert int(ws.status[_lib.ST_ANG_OVERFLOW]) == 0
     np.testing.assert_allclose(f[1], f[0], atol=1e-5 * np.abs(f[0]).max(), rtol=0)
     np.testing.assert_allclose(v[1], v[0], atol=1e-6 * np.abs(v[0]).max(), rtol=0)
+
+
+@pytest.mark.parametrize("sizes", [[1], [1024], [1025, 0, 1023], [40000], [7] * 9 + [3000], [33 * 1024 + 1] * 3])
+def test_sums_per_system(cuda_device, sizes):
+    """Energies and virials summed per system: one and several chunks of 1024, more
+    partials than a warp's 32, a warp or a thread per system, empty systems.
+
+    Bound: n float64 additions of either sign round to n 2^-53 of the sum of moduli."""
+    from fennol_b200 import _lib
+    from fennol_b200._lib import call
+
+    rng = np.random.default_rng(sum(sizes))
+    n, nsys = sum(sizes), len(sizes)
+    start = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    e = rng.standard_normal(n + 5).astype(np.float32)
+    row = rng.permutation(n + 5)[:n].astype(np.int32)
+    vir = rng.standard_normal((n, 9)).astype(np.float32)
+    dev = [torch.tensor(a, device=cuda_device) for a in (e, row, start, vir)]
+    st = torch.cuda.current_stream().cuda_stream
+    ws = torch.zeros(int(_lib.load().fennol_energy_workspace_bytes(n, nsys)), dtype=torch.uint8, device=cuda_device)
+    for name in ("fennol_energy_reduce", "fennol_energy_reduce_behind_adjoint"):
+        energy = torch.zeros(nsys, dtype=torch.float64, device=cuda_device)
+        e_atom = torch.zeros(n, dtype=torch.float64, device=cuda_device)
+        call(name, dev[0].data_ptr(), dev[1].data_ptr(), n, dev[2].data_ptr(), nsys, 0.5, energy.data_ptr(),
+             e_atom.data_ptr(), ws.data_ptr(), ws.numel(), st)
+        v = torch.zeros((nsys, 9), dtype=torch.float64, device=cuda_device)
+        call("fennol_virial_reduce", dev[3].data_ptr(), n, dev[2].data_ptr(), nsys, 0.5, v.data_ptr(), st)
+        np.testing.assert_array_equal(e_atom.cpu().numpy(), 0.5 * e[row].astype(np.float64))
+        for b in range(nsys):
+            i = slice(start[b], start[b + 1])
+            for got, x in ((energy[b:b + 1], e[row[i]][:, None]), (v[b], vir[i])):
+                x = 0.5 * x.astype(np.float64)
+                err = np.abs(got.cpu().numpy() - x.sum(0))
+                assert (err <= (sizes[b] + 1) * 2.0 ** -52 * np.abs(x).sum(0)).all()
+
+
+@pytest.mark.parametrize("kind,dtype", [(0, torch.float32), (1, torch.bfloat16), (2, torch.bfloat16),
+                                        (3, torch.float16)])
+@pytest.mark.parametrize("width,ld,off", [(1008, 1024, 0), (4, 4, 0), (1008, 1024, 1), (131, 134, 0), (1100, 1101, 0)])
+def test_gather_rows(cuda_device, kind, dtype, width, ld, off):
+    """Rows in atom order equal the parts converted and added by torch, aligned or not."""
+    from fennol_b200._lib import call
+
+    n, rows = 37, 50
+    gen = torch.Generator(device=cuda_device).manual_seed(kind + width)
+    parts = [torch.randn(rows * ld + off, generator=gen, device=cuda_device).to(dtype) for _ in range(2)]
+    at = torch.randperm(rows, generator=gen, device=cuda_device)[:n].int()
+    hi, lo = (p[off:].view(rows, ld) for p in parts)
+    want = hi[at.long(), :width].float()
+    if kind >= 2:
+        want = want + lo[at.long(), :width].float()
+    out = torch.full((n, width), 9.0, device=cuda_device)
+    call("fennol_aev_gather_rows", hi.data_ptr(), lo.data_ptr() if kind >= 2 else None, kind, ld, at.data_ptr(), n,
+         width, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(out, want)
