@@ -93,16 +93,18 @@ __device__ __forceinline__ void st4(float* p, float4 v, bool vec) {
 
 // NT = false: C = A @ W with W [K][N] (row stride ldw); K may be gathered
 // NT = true : C = A @ W^T with W [N][K] (row stride ldw); N may be gathered
-template <bool NT, int EPI>
+// RB = 2: a block has a whole 128-row tile; RB = 1: half of one (blockIdx.x = 2 tile
+// + half), 4 x 8 outputs per thread.
+template <bool NT, int EPI, int RB>
 __global__ void __launch_bounds__(kThreads, 4) k_sgemm(const __grid_constant__ GemmArgs g) {
   pdl_wait();
   // rows padded by 4 floats: the transposed stores of a warp hit 32 banks, and
   // 16-byte loads stay aligned
-  __shared__ __align__(16) float As[2][BK][BM + 4];
+  __shared__ __align__(16) float As[2][BK][64 * RB + 4];
   __shared__ __align__(16) float Bs[2][BK][BN + 4];
-  const int tile = blockIdx.x;
+  const int tile = RB == 2 ? blockIdx.x : blockIdx.x >> 1;
   const int n0 = blockIdx.y * BN;
-  const int row0 = g.tile_row[tile];
+  const int row0 = g.tile_row[tile] + (RB == 2 ? 0 : 64 * (blockIdx.x & 1));
   const int species = g.tile_species[tile];
   const int tid = threadIdx.x;
   const int tx = tid & 7, ty = tid >> 3;  // columns tx*4 and 32 + tx*4, rows ty*4 and 64 + ty*4
@@ -113,18 +115,19 @@ __global__ void __launch_bounds__(kThreads, 4) k_sgemm(const __grid_constant__ G
     const int grp = (g.model0 + m) * g.n_species + species;
     const float* __restrict__ A = g.A + (size_t)m * g.a_model + (size_t)row0 * g.lda;
     const float* __restrict__ W = g.W + (size_t)grp * g.w_group;
-    F2 acc[8][4];
+    F2 acc[4 * RB][4];
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int a = 0; a < 4 * RB; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) acc[a][b] = pack2(0.f, 0.f);
 
     // global -> register staging: A 128 rows x 16 k and W 16 x 64 as 16-byte loads
-    float4 ra[4], rb[2];
-    auto load_tile = [&](int step) {
+    constexpr int kAhead = RB == 2 ? 1 : 2;  // steps that loads run ahead
+    float4 ra_[kAhead][2 * RB], rb_[kAhead][2];
+    auto load_tile = [&](int step, float4 (&ra)[2 * RB], float4 (&rb)[2]) {
       const int ka = NT ? step * 16 : column(step);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int q = 0; q < 2 * RB; ++q)
         ra[q] = ld4(A + (size_t)((tid >> 2) + 32 * q) * g.lda + ka + (tid & 3) * 4, g.vec);
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -139,9 +142,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_sgemm(const __grid_constant__ G
         }
       }
     };
-    auto store_tile = [&](int buf) {
+    auto store_tile = [&](int buf, const float4 (&ra)[2 * RB], const float4 (&rb)[2]) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 2 * RB; ++q) {
         const int r = (tid >> 2) + 32 * q, k = (tid & 3) * 4;
         As[buf][k][r] = ra[q].x;
         As[buf][k + 1][r] = ra[q].y;
@@ -162,18 +165,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_sgemm(const __grid_constant__ G
       }
     };
 
-    load_tile(0);
-    store_tile(0);
-    __syncthreads();
-    for (int kt = 0; kt < g.nk; ++kt) {
-      const int buf = kt & 1;
-      if (kt + 1 < g.nk) load_tile(kt + 1);
+    auto multiply = [&](int buf) {
 #pragma unroll
       for (int kk = 0; kk < BK; ++kk) {
-        float av[8];
+        float av[4 * RB];
         F2 bv[4];
         *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
-        *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(&As[buf][kk][64 + ty * 4]);
+        if (RB == 2)
+          *reinterpret_cast<float4*>(av + 4 * (RB - 1)) =
+              *reinterpret_cast<const float4*>(&As[buf][kk][64 * (RB - 1) + ty * 4]);
         const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
         const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][kk][32 + tx * 4]);
         bv[0] = pack2(b0.x, b0.y);
@@ -181,14 +181,27 @@ __global__ void __launch_bounds__(kThreads, 4) k_sgemm(const __grid_constant__ G
         bv[2] = pack2(b1.x, b1.y);
         bv[3] = pack2(b1.z, b1.w);
 #pragma unroll
-        for (int a = 0; a < 8; ++a) {
+        for (int a = 0; a < 4 * RB; ++a) {
           const F2 aa = pack2(av[a], av[a]);
 #pragma unroll
           for (int b = 0; b < 4; ++b) fma2(acc[a][b], aa, bv[b]);
         }
       }
-      if (kt + 1 < g.nk) store_tile(buf ^ 1);
-      __syncthreads();
+    };
+    load_tile(0, ra_[0], rb_[0]);
+    store_tile(0, ra_[0], rb_[0]);
+    if (kAhead == 2 && g.nk > 1) load_tile(1, ra_[kAhead - 1], rb_[kAhead - 1]);
+    __syncthreads();
+    for (int kt = 0; kt < g.nk; kt += kAhead) {
+#pragma unroll
+      for (int h = 0; h < kAhead; ++h) {  // register set h: step kt + h, then step kt + h + kAhead
+        const int step = kt + h, buf = step & 1;
+        if (step >= g.nk) break;
+        if (step + kAhead < g.nk) load_tile(step + kAhead, ra_[h], rb_[h]);
+        multiply(buf);
+        if (step + 1 < g.nk) store_tile(buf ^ 1, ra_[(h + 1) % kAhead], rb_[(h + 1) % kAhead]);
+        __syncthreads();
+      }
     }
 
 #pragma unroll
@@ -199,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_sgemm(const __grid_constant__ G
       float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
       if (EPI == EPI_BIAS_CELU) bias = ld4(g.bias + (size_t)grp * g.b_group + n, g.vec);
 #pragma unroll
-      for (int a = 0; a < 8; ++a) {
+      for (int a = 0; a < 4 * RB; ++a) {
         const int r = row0 + (a < 4 ? ty * 4 + a : 64 + ty * 4 + a - 4);
         float* c = g.C + (size_t)m * g.c_model + (size_t)r * g.ldc + col;
         const float2 v0 = unpack2(acc[a][2 * h]), v1 = unpack2(acc[a][2 * h + 1]);
@@ -308,6 +321,22 @@ int models_per_launch(int rows, int n_models) {
   return std::min(n_models, std::max(1, 2400 / (3 * tiles)));
 }
 
+// One layer: half tiles where whole ones give the GPU too few blocks to be busy
+// (kFewBlocks).  An element's FMAs come in the same order either way.
+// Half tiles also load two steps ahead (128 registers hold it).  256 molecules, 1
+// model, 56 tiles, whole / half tiles: 256 -> 192 41 / 31 us, 192 -> 160 37 / 28,
+// their transposes 43 / 29 and 42 / 35; 1008 -> 256, 448 half blocks of which
+// four SMs have one more than the others, 123 / 125.
+constexpr int kFewBlocks = 148 * 4;
+template <bool NT, int EPI>
+int sgemm(int ntiles, int ny, int nz, const GemmArgs& a, cudaStream_t st) {
+  if (ntiles * ny * nz >= kFewBlocks)
+    FNL_LAUNCH_PDL((k_sgemm<NT, EPI, 2>), dim3(ntiles, ny, nz), dim3(kThreads), 0, st, a);
+  else
+    FNL_LAUNCH_PDL((k_sgemm<NT, EPI, 1>), dim3(2 * ntiles, ny, nz), dim3(kThreads), 0, st, a);
+  return FENNOL_OK;
+}
+
 }  // namespace
 
 size_t fnl_mlp_simt_workspace(int rows, const fennol_mlp_weights* w) {
@@ -372,7 +401,7 @@ int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_
         }
       }
       a.nn = d[l + 1] / 16;
-      FNL_LAUNCH_PDL((k_sgemm<false, EPI_BIAS_CELU>), dim3(ntiles, (d[l + 1] + BN - 1) / BN, nm), dim3(kThreads), 0, st, a);
+      if (int err = sgemm<false, EPI_BIAS_CELU>(ntiles, (d[l + 1] + BN - 1) / BN, nm, a, st)) return err;
     }
     // head: energy + G3 (in place of H3)
     FNL_LAUNCH_PDL(k_head, dim3((ntiles * 128 * 32 + 255) / 256), dim3(256), 0, st, Hs[3], (size_t)rows * d[3], d[3],
@@ -393,7 +422,7 @@ int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_
       a.ldc = d[l];
       a.nk = d[l + 1] / 16;
       a.nn = d[l] / 16;
-      FNL_LAUNCH_PDL((k_sgemm<true, EPI_DCELU>), dim3(ntiles, (d[l] + BN - 1) / BN, nm), dim3(kThreads), 0, st, a);
+      if (int err = sgemm<true, EPI_DCELU>(ntiles, (d[l] + BN - 1) / BN, nm, a, st)) return err;
     }
     // input gradient dX (+)= G1 W1^T / n_models
     GemmArgs a = base;
@@ -419,11 +448,11 @@ int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_
       p.C = Hs[2];
       p.c_model = (size_t)rows * N;
       p.ldc = N;
-      FNL_LAUNCH_PDL((k_sgemm<true, EPI_STORE>), dim3(ntiles, (N + BN - 1) / BN, nm), dim3(kThreads), 0, st, p);
+      if (int err = sgemm<true, EPI_STORE>(ntiles, (N + BN - 1) / BN, nm, p, st)) return err;
       FNL_LAUNCH_PDL(k_dx_sum, dim3(ntiles, (BM * N / 4 + 255) / 256), dim3(256), 0, st, a, (const float*)Hs[2], (size_t)rows * N);
       continue;
     }
-    FNL_LAUNCH_PDL((k_sgemm<true, EPI_SCALE_ACC>), dim3(ntiles, (a.nn * 16 + BN - 1) / BN), dim3(kThreads), 0, st, a);
+    if (int err = sgemm<true, EPI_SCALE_ACC>(ntiles, (a.nn * 16 + BN - 1) / BN, 1, a, st)) return err;
   }
   return FENNOL_OK;
 }

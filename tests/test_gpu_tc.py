@@ -317,3 +317,36 @@ def test_fp32_form_takes_buffers_off_16_bytes(cuda_device, groups):
         torch.cuda.synchronize()
         got.append((e_rows.cpu().numpy(), dx[off:off + ws.x.numel()].cpu().numpy()))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("atoms,models", [(1, 1), (129, 1), (700, 3)])
+def test_fp32_half_tiles_match_whole(cuda_device, atoms, models):
+    """The FP32 form in half tiles (few row tiles) gives what whole tiles give (the
+    same rows repeated until the blocks are many): every element is the same
+    chain of FMAs, so the same bits."""
+    from fennol_b200._lib import call
+    from fennol_b200.potential import C_ptr
+
+    pot = ANIPotential(precision="fp32", device=cuda_device, seed=4, n_models=models)
+    d0, F = pot.mlp.dims[0], pot.aev_cfg.aev_length
+    tiles = -(-atoms // 128)
+    gen = torch.Generator(device=cuda_device).manual_seed(atoms)
+    x1 = torch.zeros((tiles * 128, d0), device=cuda_device)
+    x1[:atoms, :F] = torch.rand((atoms, F), generator=gen, device=cuda_device)
+    got = []
+    for copies in (1, -(-600 // tiles)):
+        n = tiles * copies
+        x = x1.repeat(copies, 1).contiguous()
+        sp = torch.zeros(n, dtype=torch.int32, device=cuda_device)
+        row = torch.arange(n, dtype=torch.int32, device=cuda_device) * 128
+        e, dx = torch.zeros(n * 128, device=cuda_device), torch.zeros_like(x)
+        from fennol_b200 import _lib
+        ws = torch.zeros(int(_lib.load().fennol_mlp_workspace_bytes(pot.precision, n * 128, models, C_ptr(pot.mlp.struct))),
+                         dtype=torch.uint8, device=cuda_device)
+        call("fennol_mlp_energy_grad_groups", pot.precision, n * 128, n, sp.data_ptr(), row.data_ptr(),
+             C_ptr(pot.mlp.struct), x.data_ptr(), None, None, None, 0, e.data_ptr(), dx.data_ptr(), ws.data_ptr(),
+             ws.numel(), torch.cuda.current_stream().cuda_stream)
+        got.append((e[:atoms].cpu().numpy(), dx[:atoms].cpu().numpy()))
+    for a, b in zip(*got):
+        assert np.abs(a).max() > 0
+        np.testing.assert_array_equal(a, b)
