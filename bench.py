@@ -207,12 +207,13 @@ def time_mlp(pot, eng, reps):
 
     lay, ws = eng.layout, eng.ws
     st = torch.cuda.current_stream().cuda_stream
+    groups = pot.active_groups(lay.species_mask)
 
     def launch():
-        call("fennol_mlp_energy_grad_active", pot.precision, lay.rows, lay.ntiles, lay.t_tile_species.data_ptr(),
+        call("fennol_mlp_energy_grad_groups", pot.precision, lay.rows, lay.ntiles, lay.t_tile_species.data_ptr(),
              lay.t_tile_row.data_ptr(), C_ptr(pot.mlp.struct), ws.x.data_ptr(), _ptr(ws.x_lo),
-             pot.active_chunks(lay.species_mask), ws.e_rows.data_ptr(), ws.dx.data_ptr(), ws.mlp_ws.data_ptr(),
-             ws.mlp_ws.numel(), st)
+             groups.ctypes.data, groups.ctypes.data, groups.size, ws.e_rows.data_ptr(), ws.dx.data_ptr(),
+             ws.mlp_ws.data_ptr(), ws.mlp_ws.numel(), st)
 
     return time_launch(launch, reps)
 
@@ -245,12 +246,15 @@ def kernel_times(pot, eng, reps=20):
     st = torch.cuda.current_stream().cuda_stream
     lp = C_ptr(pot.params)
 
+    groups = pot.active_groups(lay.species_mask)
+
     # the staged pair, as the MD step launches it
     def aev_fwd():
-        call("fennol_aev_forward_staged", ws.xyzs.data_ptr(), lay.n, lay.t_atom_sys.data_ptr(),
+        call("fennol_aev_forward_groups", ws.xyzs.data_ptr(), lay.n, lay.t_atom_sys.data_ptr(),
              lay.t_cell.data_ptr(), g.rad_j.data_ptr(), g.rad_s.data_ptr(), g.rad_n.data_ptr(), g.cap_r, lp,
              lay.t_atom_row.data_ptr(), ws.aev_kind, ws.x.data_ptr(), _ptr(ws.x_lo), ws.x.shape[1],
-             g.aev_stage.data_ptr(), g.aev_stage.numel(), ws.status.data_ptr(), st)
+             groups.ctypes.data, groups.size, g.aev_stage.data_ptr(), g.aev_stage.numel(), ws.forces4.data_ptr(),
+             ws.status.data_ptr(), st)
 
     def aev_bwd():
         call("fennol_aev_backward_staged", ws.xyzs.data_ptr(), lay.n, lay.t_atom_sys.data_ptr(),
@@ -309,14 +313,14 @@ def mlp_work(pot, species, precision):
     """FLOPs per atom and model: the dense count over all 1008 AEV inputs
     (2 FLOPs per multiply-add of every layer), the count on the AEV columns that can be non-zero for
     these species, and the MMA work the fused kernel issues (padded widths,
-    active 64-column input chunks, split products)."""
+    active 16-column input groups, split products)."""
     cols = present_aev_columns(species, pot.aev_cfg)
     present = 2 * (cols * 256 + 256 * 192 + 192 * 160 + 160) * 2
     out = {"dense_flop": MLP_FLOP_PER_ATOM, "present_column_flop": present, "present_columns": cols}
     if precision in PRODUCTS:
         pf, pb = PRODUCTS[precision]
-        mask = pot.active_chunks(int(np.bitwise_or.reduce(1 << np.unique(pot.aev_cfg.species_index(species)))))
-        k1 = 64 * bin(mask & 0xFFFF).count("1")
+        mask = int(np.bitwise_or.reduce(1 << np.unique(pot.aev_cfg.species_index(species))))
+        k1 = 16 * sum(bin(int(word)).count("1") for word in pot.active_groups(mask))
         d1, d2, d3 = pot.mlp.dims[1:4]
         out["mma_flop"] = 2 * (pf * (k1 * d1 + d1 * d2 + d2 * d3) + pb * (d3 * d2 + d2 * d1 + d1 * k1))
         out["active_input_columns"] = k1
@@ -351,7 +355,7 @@ def rooflines(pot, eng, box, workload, precision, sm_mhz):
                 "flop_accounting": ("achieved = dense 1.352 MFLOP per atom and model (1008 inputs); "
                                     "present_column_tflops counts only the AEV columns these species can "
                                     "make non-zero; mma_tflops is the tensor-core work issued (padded "
-                                    "widths, active input chunks, split products)"),
+                                    "widths, active input groups, split products)"),
                 "present_column_tflops": work["present_column_flop"] * units / (kt["mlp"] * 1e-3) / 1e12},
     }
     if "mma_flop" in work:
