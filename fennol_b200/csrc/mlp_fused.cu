@@ -496,7 +496,8 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
     // each GEMM but L1 is the other region, where the epilogue has put it over
     // the accumulator it came from.  So a region is overwritten only by a GEMM
     // whose own A operand was made from the result of the last reader; what that
-    // leaves open (the next item's L1 and L2, B1 halves) is waited for.
+    // leaves open (the next item's L1 and L2, B1 halves) is waited for, and so is
+    // what it leaves open about the barriers (the next item's L1).
     const bool leader = elect_one();
     uint32_t seq = 0, pos = 0;      // next chunk and its place in the ring
     uint32_t act_par = 0;           // parity of the atoms' next phases
@@ -586,6 +587,11 @@ k_mlp_fused(const __grid_constant__ Maps maps, const __grid_constant__ FusedPara
           give();
         }
         if (!ok) break;
+        // The two accumulator barriers take turns, and a phase must not complete
+        // while a warp still waits for the one before it.  L1's was last used by
+        // the item before: by B2 after one run, else by its run before the last,
+        // which every warp has taken once it has read it.
+        if (p.ndx > kRunGroups && !(ok = dx_read(runs & 1))) break;
         finish();
       }
       // L2, L3, B3, B2

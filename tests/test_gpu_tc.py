@@ -350,3 +350,66 @@ def test_fp32_half_tiles_match_whole(cuda_device, atoms, models):
     for a, b in zip(*got):
         assert np.abs(a).max() > 0
         np.testing.assert_array_equal(a, b)
+
+
+def _tile_batch(pot, tiles, columns, seed, species=None):
+    """AEV rows of ``tiles`` full row tiles, random in the given columns and zero
+    elsewhere, in the form's operand layout; the tiles' species and first rows."""
+    dev, d0 = pot.device, pot.mlp.dims[0]
+    gen = torch.Generator(device=dev).manual_seed(seed)
+    x = torch.zeros((tiles * 128, d0), device=dev)
+    x[:, columns] = torch.rand((tiles * 128, len(columns)), generator=gen, device=dev)
+    half = torch.float16 if pot.precision_name.startswith("f16") else torch.bfloat16
+    hi = x.to(half)
+    lo = (x - hi.float()).to(half)
+    if species is None:
+        species = pot.mlp.n_species
+    sp = torch.arange(tiles, dtype=torch.int32, device=dev) % species
+    return hi, lo, sp, torch.arange(tiles, dtype=torch.int32, device=dev) * 128
+
+
+def _tile_results(pot, batch, ws, x_groups=None, dx_groups=None):
+    """Row energies and dE/dAEV of a ``_tile_batch``, into buffers filled with a marker."""
+    from fennol_b200._lib import call
+    from fennol_b200.potential import C_ptr
+
+    hi, lo, sp, row = batch
+    n = sp.numel()
+    e = torch.full((n * 128,), 7.0, device=pot.device)
+    dx = torch.full(hi.shape, 7.0, device=pot.device)
+    words = 0 if x_groups is None and dx_groups is None else pot.mlp.dims[0] // 1024
+    call("fennol_mlp_energy_grad_groups", pot.precision, n * 128, n, sp.data_ptr(), row.data_ptr(),
+         C_ptr(pot.mlp.struct), hi.data_ptr(), lo.data_ptr(), None if x_groups is None else x_groups.ctypes.data,
+         None if dx_groups is None else dx_groups.ctypes.data, words, e.data_ptr(), dx.data_ptr(), ws.data_ptr(),
+         ws.numel(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert int(ws[:4].view(torch.int32)[0]) == 0  # no wait ran out
+    return e, dx
+
+
+def _tile_workspace(pot, tiles):
+    from fennol_b200 import _lib
+    from fennol_b200.potential import C_ptr
+
+    nb = _lib.load().fennol_mlp_workspace_bytes(pot.precision, tiles * 128, pot.mlp.n_models, C_ptr(pot.mlp.struct))
+    return torch.zeros(int(nb), dtype=torch.uint8, device=pot.device)
+
+
+@pytest.mark.parametrize("precision,wanted,models", [("f16x3x1", 64, 1), ("bf16", 64, 3), ("f16x3x2", 24, 1),
+                                                     ("bf16x2", 9, 2)])
+def test_short_first_layer_behind_many_dx_runs(cuda_device, precision, wanted, models):
+    """A first layer of one column group right behind the 2 to 8 dX runs of the
+    item before: its accumulator is announced on the barrier of the run before
+    the last, which every epilogue warp must have taken by then.  Same bits as
+    with every input column (the others are zero)."""
+    pot = ANIPotential(precision=precision, device=cuda_device, seed=2, n_models=models)
+    tiles = 3 * torch.cuda.get_device_properties(cuda_device).multi_processor_count + 80
+    batch = _tile_batch(pot, tiles, np.arange(16), seed=wanted)
+    ws = _tile_workspace(pot, tiles)
+    one = np.array([1], np.uint64)
+    want = np.array([2 ** wanted - 1], np.uint64)
+    e, dx = _tile_results(pot, batch, ws, None, want)
+    assert float(dx[:, :16 * wanted].abs().max()) > 0
+    for _ in range(20):
+        e1, dx1 = _tile_results(pot, batch, ws, one, want)
+        assert torch.equal(e1, e) and torch.equal(dx1, dx)
