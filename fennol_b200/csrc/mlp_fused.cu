@@ -977,7 +977,8 @@ __global__ void __launch_bounds__(kJoinThreads) k_mlp_join(const __grid_constant
   if (i >= p.ndx) return;
   const float4* xs = reinterpret_cast<const float4*>(p.xs) + (size_t)(i * 4 + j) * BM + r;
   const size_t per = (size_t)p.ndx * 4 * BM;
-  // slot of the k-th summand: model k, or part k (the CTAs from the tile's first on)
+  // slot of the k-th summand: model k, or part k (the CTAs from the tile's first on,
+  // each of which has items then)
   const int c0 = share.owner(t0);
   const int n = p.apart ? M : share.owner(t0 + M - 1) - c0 + 1;
   __shared__ int slots[kJoinThreads];
@@ -1097,11 +1098,15 @@ size_t dc_bytes(int grid, const fennol_mlp_weights* w) {
 }
 // Up to 16 dX column groups the models of a shared tile are kept apart, so that
 // its sum does not depend on how it was shared; wider rows are summed part by
-// part (kept apart, 256 molecules x 8 models would move 0.23 GB more).
+// part (kept apart, 256 molecules x 8 models would move 0.23 GB more).  Parts need
+// an item for every CTA: with fewer items than CTAs those without one lie among
+// the owners of a tile's items, and their slots hold something else.  There a CTA
+// has one item at most, so that keeping the models apart takes no more slots.
 constexpr int kApartGroups = 16;
+bool models_apart(const Share& share, int ndx) { return ndx <= kApartGroups || share.most() <= 1; }
 int xs_slots(const Share& share, int ndx, int n_models) {
   if (n_models == 1) return 0;
-  return std::max(1, ndx <= kApartGroups ? share.most() : std::min(share.most(), 2));
+  return std::max(1, models_apart(share, ndx) ? share.most() : std::min(share.most(), 2));
 }
 // for any number of tiles up to `tiles`
 size_t xs_bytes(int tiles, int grid, const fennol_mlp_weights* w) {
@@ -1233,7 +1238,7 @@ int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, 
   p.e_part = (float*)((char*)p.xs + xs_bytes(ntiles, grid, w));
   const Share share(ntiles, w->n_models, grid);
   p.xs_slots = xs_slots(share, p.ndx, w->n_models);
-  p.apart = p.ndx <= kApartGroups;
+  p.apart = models_apart(share, p.ndx);
   FNL_LAUNCH_PDL(kern, dim3(grid), dim3(kThreads), smem, st, maps, p);
   FNL_CHECK_LAUNCH();
   if (w->n_models > 1 && share.left > 0) {

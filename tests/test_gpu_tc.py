@@ -413,3 +413,32 @@ def test_short_first_layer_behind_many_dx_runs(cuda_device, precision, wanted, m
     for _ in range(20):
         e1, dx1 = _tile_results(pot, batch, ws, one, want)
         assert torch.equal(e1, e) and torch.equal(dx1, dx)
+
+
+@pytest.mark.parametrize("precision", ["f16x3x1", "bf16x2"])
+@pytest.mark.parametrize("extra,models", [(1, 8), (2, 2), (2, 5), (18, 8), (19, 8), (72, 2), (74, 2), (149, 3)])
+def test_join_adds_only_what_the_tile_has(cuda_device, precision, extra, models):
+    """Tiles beyond a whole number per CTA, seven species and every column of dX
+    wanted: shared tiles with fewer items than CTAs (most of them have none of
+    the tile), as many, and more.  The scratch holds a marker before the call.
+    dE/dAEV and the energies are the mean of the single-model results: float32
+    sums of at most eight terms, 8 half-ulps of the largest one."""
+    W = init_weights(CFG, MCFG, seed=3, n_models=models)
+    if precision == "bf16x2":
+        W = round_weights_bf16(W)
+    pot = ANIPotential(precision=precision, device=cuda_device, weights=W)
+    tiles = torch.cuda.get_device_properties(cuda_device).multi_processor_count + extra
+    batch = _tile_batch(pot, tiles, np.arange(CFG.aev_length), seed=extra)
+    ws = _tile_workspace(pot, tiles)
+    ws[256:] = 0x7F  # 3.4e38 as float32
+    e, dx = _tile_results(pot, batch, ws)
+    es, ds, em, dm = 0.0, 0.0, 0.0, 0.0
+    for m in range(models):
+        one = ANIPotential(precision=precision, device=cuda_device, weights=[W[m]])
+        e1, d1 = _tile_results(one, batch, _tile_workspace(one, tiles))
+        es, ds = max(es, float(e1.abs().max())), max(ds, float(d1.abs().max()))
+        em, dm = em + e1.double() / models, dm + d1.double() / models
+    tol = 8 * 2.0 ** -24
+    assert ds > 0
+    assert float((e.double() - em).abs().max()) <= tol * es
+    assert float((dx.double() - dm).abs().max()) <= tol * ds
