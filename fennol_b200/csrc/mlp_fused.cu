@@ -1144,6 +1144,10 @@ int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, 
   if (f16 && (!w->wt_lo[0] || !w->wt_lo[1] || !w->wt_lo[2])) return FENNOL_ERR_INVALID;
   if (wblo && (!w->w_lo[0] || !w->w_lo[1] || !w->w_lo[2])) return FENNOL_ERR_INVALID;
   if (f16 && ((uintptr_t)w->f16_scale & 15) != 0) return FENNOL_ERR_INVALID;
+  // bulk copies bring them to shared memory; a group's start is aligned where the
+  // array is (widths are multiples of 64)
+  if ((((uintptr_t)w->b32[0] | (uintptr_t)w->b32[1] | (uintptr_t)w->b32[2] | (uintptr_t)w->w32[3]) & 15) != 0)
+    return FENNOL_ERR_INVALID;
   FusedParams p{};
   // Column lists: the L1 units with a column that may be non-zero, and which of
   // their K steps have one

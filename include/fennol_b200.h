@@ -370,6 +370,8 @@ int fennol_aev_tangent(const float* xyzs, int natoms, const int* atom_sys, const
  * power of two applied to the last layer's kernel inside the input-gradient
  * GEMMs.  wt_lo is required for both FP16 forms, w_lo for F16X3X2 only.
  * f16_scale (16-byte aligned) may be NULL for the other forms.
+ * The fused tensor-core kernel wants b32[0..2] and w32[3] 16-byte aligned
+ * (FENNOL_ERR_INVALID otherwise).
  */
 typedef struct fennol_mlp_weights {
   int n_models;

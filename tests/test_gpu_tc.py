@@ -442,3 +442,23 @@ def test_join_adds_only_what_the_tile_has(cuda_device, precision, extra, models)
     assert ds > 0
     assert float((e.double() - em).abs().max()) <= tol * es
     assert float((dx.double() - dm).abs().max()) <= tol * ds
+
+
+@pytest.mark.parametrize("field", ["b32", "w32"])
+def test_fused_form_refuses_biases_off_16_bytes(cuda_device, field):
+    """The fused kernel copies biases and the last kernel in bulk, which needs
+    16-byte aligned addresses: others are refused before anything is launched."""
+    import ctypes
+
+    from fennol_b200 import _lib
+
+    pot = ANIPotential(precision="f16x3x1", device=cuda_device, seed=0)
+    batch, ws = _tile_batch(pot, 1, np.arange(16), seed=1, species=1), _tile_workspace(pot, 1)
+    _tile_results(pot, batch, ws)
+    good = _lib.MLPWeights.from_buffer_copy(pot.mlp.struct)
+    for l in ([0, 1, 2] if field == "b32" else [3]):
+        getattr(pot.mlp.struct, field)[l] += 4
+        with pytest.raises(_lib.FennolError):
+            _tile_results(pot, batch, ws)
+        ctypes.memmove(ctypes.byref(pot.mlp.struct), ctypes.byref(good), ctypes.sizeof(good))
+    _tile_results(pot, batch, ws)
