@@ -632,7 +632,9 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   pdl_wait();
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
-  const int i = min(warp, n - 1);  // the warps past the last row do it once more
+  // the warps past the last row stay for the block's report: no entries, no writes
+  const bool row = warp < n;
+  const int i = row ? warp : n - 1;
   int b = atom_sys[i];
   const float* c = sys_cell ? sys_cell + 9 * b : nullptr;
   auto position = [&](int k) {
@@ -641,7 +643,7 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
   };
   const float4 pi = position(i);
   const int seen = status_peek(status, ST_FILTER_MAXCOUNT);
-  int cnt = in_count[i];
+  int cnt = row ? in_count[i] : 0;
   if (cnt > in_cap) cnt = in_cap;
   size_t ib = (size_t)i * in_cap, ob = (size_t)i * out_cap;
   int count = 0;
@@ -690,7 +692,7 @@ k_filter(const float* __restrict__ coords, int n, const int* __restrict__ atom_s
       count += __popc(m);
     }
   }
-  if (lane == 0) {
+  if (row && lane == 0) {
     out_count[i] = count < out_cap ? count : out_cap;
     if (count > out_cap) status_set(status, ST_FILTER_OVERFLOW);
   }

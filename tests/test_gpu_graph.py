@@ -279,3 +279,33 @@ def test_packed_filter_matches_plain(pot, cuda_device, n_side, skin, cap):
     assert words[_lib.ST_NBR_OVERFLOW] == 0 and words[_lib.ST_FILTER_OVERFLOW] == 0
     assert words[_lib.ST_NBR_MAXCOUNT] == int(g.nbr_n.max()) > 0
     assert words[_lib.ST_FILTER_MAXCOUNT] == rows[0][2].max() > 0
+
+
+@pytest.mark.parametrize("atoms", [1, 2, 9, 15, 17])
+@pytest.mark.parametrize("packed", [False, True])
+def test_filter_writes_each_row_once(pot, cuda_device, atoms, packed):
+    """A list filtered into itself (each row has one warp, which has read an entry
+    before the place is written again): with any other warp on the last row, that
+    row could be filtered once more from what is left of it."""
+    s = water_box(6, seed=4)
+    xyz, sp = s.coordinates[:atoms], s.species[:atoms]
+    lay = pot.layout(sp, [atoms])
+    coords = torch.tensor(xyz, dtype=torch.float32, device=cuda_device)
+    pos = torch.zeros((atoms, 4), device=cuda_device)
+    pos[:, :3] = coords
+    cap = 40
+    status = torch.zeros(8, dtype=torch.int32, device=cuda_device)
+    st = torch.cuda.current_stream().cuda_stream
+    g = GraphBuffers(lay, 3.0, 9.0, cap, cap)
+    g.build(lay, coords, status, st)
+    g.filter(lay, pos if packed else coords, status, st)
+    want = [g.rad_n.clone()] + [torch.where(torch.arange(cap, device=cuda_device) < g.rad_n[:, None], t, 0)
+                                for t in (g.rad_j, g.rad_s)]
+    for _ in range(20):
+        g2 = GraphBuffers(lay, 3.0, 9.0, cap, cap)
+        g2.build(lay, coords, status, st)
+        g2.rad_j, g2.rad_s, g2.rad_n = g2.nbr_j, g2.nbr_s, g2.nbr_n
+        g2.filter(lay, pos if packed else coords, status, st)
+        got = [g2.rad_n] + [torch.where(torch.arange(cap, device=cuda_device) < g2.rad_n[:, None], t, 0)
+                            for t in (g2.rad_j, g2.rad_s)]
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
