@@ -313,12 +313,12 @@ __global__ void __launch_bounds__(256) k_head(float* __restrict__ H3, size_t h_m
 }
 
 // Models evaluated per launch: as many as give 2,400 blocks of the narrower
-// layers, four waves of the GPU, so that a nearly empty last wave costs little
-// (6,591 atoms x 8 models in two launches of 624 blocks, 1.05 waves: 90 us
-// each); the activations in memory stay below those of about 100,000 rows.
+// layers (three a tile), four waves of the GPU, so that a nearly empty last wave
+// costs little (6,591 atoms x 8 models in two launches of 624 blocks, 1.05 waves:
+// 90 us each); the activations in memory stay below those of about 100,000 rows.
+constexpr int kLaunchTiles = 800;  // (tile, model) pairs per launch
 int models_per_launch(int rows, int n_models) {
-  const int tiles = std::max(rows / BM, 1);
-  return std::min(n_models, std::max(1, 2400 / (3 * tiles)));
+  return std::min(n_models, std::max(1, kLaunchTiles / std::max(rows / BM, 1)));
 }
 
 // One layer: half tiles where whole ones give the GPU too few blocks to be busy
@@ -339,8 +339,12 @@ int sgemm(int ntiles, int ny, int nz, const GemmArgs& a, cudaStream_t st) {
 
 }  // namespace
 
+// Activations of a launch: those of `rows` or of any fewer rows, which can be
+// more (100 tiles go through 8 models at a time, 101 through 7).
 size_t fnl_mlp_simt_workspace(int rows, const fennol_mlp_weights* w) {
-  return (size_t)models_per_launch(rows, w->n_models) * rows * (w->dims[1] + w->dims[2] + w->dims[3]) * sizeof(float);
+  const size_t tiles = ((size_t)rows + BM - 1) / BM;
+  const size_t most = std::min(tiles * w->n_models, std::max(tiles, (size_t)kLaunchTiles));
+  return most * BM * (w->dims[1] + w->dims[2] + w->dims[3]) * sizeof(float);
 }
 
 int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_row,

@@ -387,7 +387,10 @@ typedef struct fennol_mlp_weights {
   const float* f16_scale;
 } fennol_mlp_weights;
 
-/* Workspace of fennol_mlp_energy_grad for `rows` padded rows, in bytes. */
+/*
+ * Workspace of fennol_mlp_energy_grad for `rows` padded rows, in bytes: enough
+ * for fewer rows too.
+ */
 size_t fennol_mlp_workspace_bytes(int precision, int rows, int n_models,
                                   const fennol_mlp_weights* w);
 

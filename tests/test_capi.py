@@ -151,3 +151,21 @@ def test_aev_active_chunks_cover_every_nonzero_column():
         assert all((chunks >> (c // 64)) & 1 for c in nz), (mask, bin(chunks))
         assert chunks & ~lib.fennol_aev_active_chunks(C_ptr(p), 0x7F) == 0
     assert lib.fennol_aev_active_chunks(C_ptr(p), 0x7F) == (1 << 16) - 1
+
+
+@pytest.mark.parametrize("precision", sorted(_lib.PRECISIONS))
+@pytest.mark.parametrize("models", [1, 2, 5, 8])
+def test_mlp_workspace_never_shrinks_with_the_rows(precision, models):
+    """A workspace sized for a caller's largest batch serves its smaller ones."""
+    w = _lib.MLPWeights()
+    w.n_models, w.n_species, w.celu_alpha = models, 7, 0.1
+    for k, d in enumerate([1024, 256, 192, 192, 1]):
+        w.dims[k] = d
+    w.f16_scale = 16  # never followed
+    lib = _lib.load()
+    got = [lib.fennol_mlp_workspace_bytes(_lib.PRECISIONS[precision], 128 * t, models, C.byref(w))
+           for t in range(1, 1200)]
+    assert got[0] > 0 and all(a <= b for a, b in zip(got, got[1:]))
+    if precision == "fp32":  # the activations of at most 800 (tile, model) pairs, or of one model
+        per = 128 * (256 + 192 + 192) * 4
+        assert all(g <= per * max(t, 800) for t, g in enumerate(got, 1))
