@@ -372,9 +372,9 @@ class Workspace:
             self.aev_kind = _lib.AEV_BF16 if pot.precision == _lib.MLP_BF16 else _lib.AEV_BF16X2
         self.dx = torch.zeros((rows, d0), dtype=torch.float32, device=dev)
         self.e_rows = torch.zeros(rows, dtype=torch.float32, device=dev)
-        mws = _lib.load().fennol_mlp_workspace_bytes(pot.precision, rows, pot.mlp.n_models,
-                                                     pot.mlp.struct)
-        self.mlp_ws = torch.zeros(max(int(mws), 256), dtype=torch.uint8, device=dev)
+        # scratch that is written before it is read, behind the MLP's error word
+        self.mlp_ws = torch.empty(pot.mlp_workspace_bytes(rows), dtype=torch.uint8, device=dev)
+        self.mlp_ws[:256].zero_()
         self.forces4 = torch.zeros((n, 4), dtype=torch.float32, device=dev)
         self.forces = torch.zeros((n, 3), dtype=torch.float32, device=dev)
         self.energy = torch.zeros(layout.nsys, dtype=torch.float64, device=dev)
@@ -500,6 +500,11 @@ class ANIPotential:
             call("fennol_aev_active_groups", C_ptr(self.params), species_mask, words.ctypes.data, words.size)
             self._group_masks[species_mask] = words
         return words
+
+    def mlp_workspace_bytes(self, rows: int) -> int:
+        """Device bytes of the MLP's scratch for ``rows`` padded rows."""
+        return max(256, int(_lib.load().fennol_mlp_workspace_bytes(self.precision, rows, self.mlp.n_models,
+                                                                   self.mlp.struct)))
 
     def mlp_launches(self, ntiles: Optional[int] = None) -> int:
         """Kernels launched by one MLP call: the FP32 form runs 7 per

@@ -45,7 +45,7 @@ from . import _lib
 from ._lib import call
 from .md import KB_KCALMOL, MASS_DA_TO_MD, launch_flagged_rebuild
 from .params import atomic_masses
-from .potential import (MAX_ROW, ANIPotential, BatchLayout, GraphBuffers, HARTREE_TO_KCALMOL,
+from .potential import (MAX_ROW, TILE, ANIPotential, BatchLayout, GraphBuffers, HARTREE_TO_KCALMOL,
                         Workspace, _ptr, min_image_ok)
 
 
@@ -143,7 +143,7 @@ class _EFLane:
             ev = torch.cuda.Event()
             ev.record(self.stream)
         self.inflight = dict(batch=b, coords=coords, g=g, ws=ws, h_e=h_e, h_f=h_f, h_st=h_st, ev=ev,
-                             bytes=e.bytes_per_atom * b.n)
+                             bytes=e.batch_bytes(b.n, e.bytes_per_atom))
         e.bytes_in_flight += self.inflight["bytes"]
 
     def _evaluate(self, b: _Batch, coords, g: GraphBuffers, ws: Workspace, st: int):
@@ -353,7 +353,7 @@ class _MDLane:
                     self.members, self.state = [], None
                     return False
                 st, members = self._new_state(keep, admit, batch)
-                st["bytes"] = e.bytes_per_atom_md * st["batch"].n
+                st["bytes"] = e.batch_bytes(st["batch"].n, e.bytes_per_atom_md)
                 e.bytes_in_flight += st["bytes"]
                 self.state, self.members = st, members
                 self._build(st)
@@ -461,10 +461,20 @@ class ServingEngine:
         # AEV rows (hi+lo or fp32) + dE/dAEV + neighbour rows + per-atom state
         self.bytes_per_atom = d0 * (act + 4) + 8 * 128 + 256
         self.bytes_per_atom_md = self.bytes_per_atom + 8 * 96 + 128
+        self._mlp_bytes: Dict[int, int] = {}
         self.bytes_in_flight = 0
         self.results: List[ServeResult] = []
         self.ef = _EFLane(self)
         self.md = _MDLane(self)
+
+    def batch_bytes(self, atoms: int, per_atom: int) -> int:
+        """Device bytes of a batch: ``per_atom`` for each atom, and the MLP's
+        scratch for its rows (every species' rows padded to a tile), which for an
+        ensemble is 190 MB from about 2,500 atoms on."""
+        tiles = atoms // TILE + min(self.pot.mlp.n_species, atoms)
+        if tiles not in self._mlp_bytes:
+            self._mlp_bytes[tiles] = self.pot.mlp_workspace_bytes(TILE * tiles)
+        return per_atom * atoms + self._mlp_bytes[tiles]
 
     def _md_admits(self, running: int, pop: bool) -> List[tuple]:
         """Ready MD requests, in order, that fit beside ``running`` atoms in
@@ -476,7 +486,7 @@ class ServingEngine:
         admit, atoms = [], running
         for item in list(md.ready):
             n_new = item[0].natoms
-            fits = n_new <= room and other + self.bytes_per_atom_md * (atoms + n_new) <= self.budget
+            fits = n_new <= room and other + self.batch_bytes(atoms + n_new, self.bytes_per_atom_md) <= self.budget
             if not fits and (admit or running or other):
                 break
             admit.append(item)
@@ -492,7 +502,8 @@ class ServingEngine:
             r = queue[0]
             if out and atoms + r.natoms > max_atoms:
                 break
-            if self.bytes_in_flight + per_atom * (atoms + r.natoms) > self.budget and (out or self.bytes_in_flight):
+            if (out or self.bytes_in_flight) and \
+                    self.bytes_in_flight + self.batch_bytes(atoms + r.natoms, per_atom) > self.budget:
                 break
             out.append(queue.popleft())
             atoms += r.natoms

@@ -95,3 +95,27 @@ def test_realtime_stream_latencies(pot):
     lat = latency_percentiles(res)
     assert 0 < lat["p50_ms"] <= lat["p99_ms"]
     assert all(r.done >= r.arrival for r in res)
+
+
+@pytest.mark.parametrize("precision,models", [("f16x3x1", 1), ("f16x3x1", 8), ("fp32", 8), ("bf16x3", 2)])
+def test_admission_counts_the_mlp_scratch(cuda_device, precision, models):
+    """A batch counts at least the bytes of its rows and of the MLP's scratch, in
+    flight and in the admission, for few atoms of many species and for many."""
+    from collections import deque
+
+    pot = ANIPotential(precision=precision, device=cuda_device, seed=0, n_models=models)
+    for systems in (molecule_batch(1, seed=3), molecule_batch(24, seed=4), [water_box(8, seed=1)]):
+        reqs = [ServeRequest(k, "ef", s.species, s.coordinates, getattr(s, "cell", None))
+                for k, s in enumerate(systems)]
+        eng = ServingEngine(pot)
+        eng.ef.launch(reqs)
+        b, ws = eng.ef.inflight["batch"], eng.ef.inflight["ws"]
+        held = ws.mlp_ws.numel() + b.n * sum(t.element_size() * t.shape[1] for t in (ws.x, ws.x_lo, ws.dx)
+                                             if t is not None)
+        assert eng.bytes_in_flight >= held
+        while not eng.ef.poll(lambda: 0.0):
+            pass
+        assert eng.bytes_in_flight == 0 and len(eng.results) == len(reqs)
+        # a budget that holds the first request and not the next beside it
+        eng.budget = eng.batch_bytes(reqs[0].natoms, eng.bytes_per_atom)
+        assert len(eng._take(deque(reqs), 1 << 20, eng.bytes_per_atom)) == 1
