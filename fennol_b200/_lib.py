@@ -118,6 +118,7 @@ _SIGNATURES = {
     "fennol_mlp_energy_grad": (I, [I, I, I, P, P, C.POINTER(MLPWeights), P, P, P, P, P, SZ, P]),
     "fennol_mlp_energy_grad_active": (I, [I, I, I, P, P, C.POINTER(MLPWeights), P, P, ULL, P, P, P, SZ, P]),
     "fennol_mlp_energy_grad_groups": (I, [I, I, I, P, P, C.POINTER(MLPWeights), P, P, P, P, I, P, P, P, SZ, P]),
+    "fennol_mlp_launches": (I, [I, I, I, C.POINTER(MLPWeights), P, I, I]),
     "fennol_aev_active_groups": (I, [C.POINTER(AEVParams), C.c_uint, P, I]),
     "fennol_aev_active_chunks": (ULL, [C.POINTER(AEVParams), C.c_uint]),
     "fennol_energy_workspace_bytes": (SZ, [I, I]),

@@ -64,6 +64,17 @@ extern "C" int fennol_mlp_energy_grad_groups(int precision, int rows, int ntiles
                      fnl::ColumnGroups{host_dx_groups}, e_rows, dx, workspace, workspace_bytes, stream);
 }
 
+extern "C" int fennol_mlp_launches(int precision, int rows, int ntiles, const fennol_mlp_weights* w,
+                                   const unsigned long long* host_dx_groups, int group_words, int want_dx) {
+  if (precision < FENNOL_MLP_FP32 || precision > FENNOL_MLP_F16X3X2 || !weights_ok(precision, w)) return FENNOL_ERR_INVALID;
+  if (rows < 0 || ntiles < 0 || rows % 128 != 0 || ntiles * 128ll > rows) return FENNOL_ERR_INVALID;
+  if (host_dx_groups && (long long)group_words * 64 * 16 < w->dims[0]) return FENNOL_ERR_INVALID;
+  if (ntiles == 0) return 0;
+  return precision == FENNOL_MLP_FP32
+             ? fnl_mlp_simt_launches(rows, ntiles, w, fnl::ColumnGroups{host_dx_groups}, want_dx != 0)
+             : fnl_mlp_tc_launches(precision, ntiles, w, want_dx != 0);
+}
+
 extern "C" int fennol_mlp_energy_grad_active(int precision, int rows, int ntiles, const int* tile_species,
                                              const int* tile_row, const fennol_mlp_weights* w, const void* x,
                                              const void* x_lo, unsigned long long active_chunks, float* e_rows,

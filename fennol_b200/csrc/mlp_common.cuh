@@ -30,12 +30,16 @@ size_t fnl_mlp_simt_workspace(int rows, const fennol_mlp_weights* w);
 int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_row,
                  const fennol_mlp_weights* w, const float* x, fnl::ColumnGroups xg, fnl::ColumnGroups dg,
                  float* e_rows, float* dx, void* ws, cudaStream_t st);
+// The *_launches functions: kernels of one call.
+int fnl_mlp_simt_launches(int rows, int ntiles, const fennol_mlp_weights* w, fnl::ColumnGroups dg, bool want_dx);
 size_t fnl_mlp_tc_workspace(int precision, int rows, int n_models, const fennol_mlp_weights* w);
 int fnl_mlp_tc(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
                const fennol_mlp_weights* w, const void* x, const void* x_lo, fnl::ColumnGroups xg,
                fnl::ColumnGroups dg, float* e_rows, float* dx, void* ws, size_t ws_bytes, cudaStream_t st);
+int fnl_mlp_tc_launches(int precision, int ntiles, const fennol_mlp_weights* w, bool want_dx);
 bool fnl_mlp_fused_supported(int precision, const fennol_mlp_weights* w);
 size_t fnl_mlp_fused_workspace(int rows, const fennol_mlp_weights* w);
 int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
                   const fennol_mlp_weights* w, const void* x, const void* x_lo, fnl::ColumnGroups xg,
                   fnl::ColumnGroups dg, float* e_rows, float* dx, void* ws, size_t ws_bytes, cudaStream_t st);
+int fnl_mlp_fused_launches(int ntiles, const fennol_mlp_weights* w);

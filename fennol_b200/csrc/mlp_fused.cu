@@ -1130,6 +1130,12 @@ size_t fnl_mlp_fused_workspace(int rows, const fennol_mlp_weights* w) {
   return 256 + 128 + dc_bytes(grid, w) + xs_bytes(rows / BM, grid, w) + e_part_bytes(rows / BM, w);
 }
 
+// The kernel, and the join of the tiles that CTAs share.
+int fnl_mlp_fused_launches(int ntiles, const fennol_mlp_weights* w) {
+  const Share share(ntiles, w->n_models, fused_grid(ntiles, w->n_models));
+  return w->n_models > 1 && share.left > 0 ? 2 : 1;
+}
+
 int fnl_mlp_fused(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
                   const fennol_mlp_weights* w, const void* x, const void* x_lo, ColumnGroups xg, ColumnGroups dg,
                   float* e_rows, float* dx, void* ws, size_t ws_bytes, cudaStream_t st) {

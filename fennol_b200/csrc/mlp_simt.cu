@@ -337,6 +337,13 @@ int sgemm(int ntiles, int ny, int nz, const GemmArgs& a, cudaStream_t st) {
   return FENNOL_OK;
 }
 
+// Few columns of dX on few tiles: a block per model, into the activations that are
+// no longer needed (H2), and a sum; 106 blocks that went through 8 models took 176
+// us on 6,591 atoms, 848 blocks and the sum 96 us.
+bool dx_by_model(int models, int ntiles, int N, const int* d) {
+  return models > 1 && ntiles * ((N + BN - 1) / BN) < kFewBlocks && N <= d[2];
+}
+
 }  // namespace
 
 // Activations of a launch: those of `rows` or of any fewer rows, which can be
@@ -345,6 +352,19 @@ size_t fnl_mlp_simt_workspace(int rows, const fennol_mlp_weights* w) {
   const size_t tiles = ((size_t)rows + BM - 1) / BM;
   const size_t most = std::min(tiles * w->n_models, std::max(tiles, (size_t)kLaunchTiles));
   return most * BM * (w->dims[1] + w->dims[2] + w->dims[3]) * sizeof(float);
+}
+
+int fnl_mlp_simt_launches(int rows, int ntiles, const fennol_mlp_weights* w, ColumnGroups dg, bool want_dx) {
+  const int per = models_per_launch(rows, w->n_models), groups = w->dims[0] / 16;
+  int wanted = 0, n = 0;
+  for (int g = 0; g < groups; ++g) wanted += groups > kMaxGroups || dg.has(g);
+  for (int m0 = 0; m0 < w->n_models; m0 += per) {
+    n += 4;  // three layers and the head
+    if (!want_dx) continue;
+    n += 2;
+    if (wanted > 0) n += 1 + dx_by_model(std::min(per, w->n_models - m0), ntiles, 16 * wanted, w->dims);
+  }
+  return n;
 }
 
 int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_row,
@@ -443,11 +463,8 @@ int fnl_mlp_simt(int rows, int ntiles, const int* tile_species, const int* tile_
     a.all = 0;
     a.nn = list(a, dg);
     if (a.nn == 0) continue;
-    const int N = a.nn * 16, blocks = ntiles * ((N + BN - 1) / BN);
-    // Few columns on few tiles: a block per model, into the activations that
-    // are no longer needed (H2), and a sum; 106 blocks that went through 8
-    // models took 176 us on 6,591 atoms, 848 blocks and the sum 96 us.
-    if (nm > 1 && blocks < 592 && N <= d[2]) {
+    const int N = a.nn * 16;
+    if (dx_by_model(nm, ntiles, N, d)) {
       GemmArgs p = a;
       p.C = Hs[2];
       p.c_model = (size_t)rows * N;

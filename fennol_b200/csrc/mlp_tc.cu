@@ -465,15 +465,26 @@ size_t fnl_mlp_tc_workspace(int precision, int rows, int n_models, const fennol_
   return a;
 }
 
+// The FP16 forms exist only as the fused kernel.
+static bool runs_fused(int precision, const fennol_mlp_weights* w) {
+  const bool f16 = precision == FENNOL_MLP_F16X3X1 || precision == FENNOL_MLP_F16X3X2;
+  return fnl_mlp_fused_supported(precision, w) && (f16 || !getenv("FENNOL_MLP_UNFUSED"));
+}
+
+int fnl_mlp_tc_launches(int precision, int ntiles, const fennol_mlp_weights* w, bool want_dx) {
+  if (runs_fused(precision, w)) return fnl_mlp_fused_launches(ntiles, w);
+  return (want_dx ? 6 : 3) * w->n_models + 1;
+}
+
 int fnl_mlp_tc(int precision, int rows, int ntiles, const int* tile_species, const int* tile_row,
                const fennol_mlp_weights* w, const void* x, const void* x_lo, ColumnGroups xg, ColumnGroups dg,
                float* e_rows, float* dx, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (!encode_fn()) return FENNOL_ERR_UNSUPPORTED;
   const bool f16 = precision == FENNOL_MLP_F16X3X1 || precision == FENNOL_MLP_F16X3X2;
-  if (fnl_mlp_fused_supported(precision, w) && (f16 || !getenv("FENNOL_MLP_UNFUSED")))
+  if (runs_fused(precision, w))
     return fnl_mlp_fused(precision, rows, ntiles, tile_species, tile_row, w, x, x_lo, xg, dg, e_rows, dx, ws,
                          ws_bytes, st);
-  if (f16) return FENNOL_ERR_UNSUPPORTED;  // the FP16 forms exist only as the fused kernel
+  if (f16) return FENNOL_ERR_UNSUPPORTED;
   const int* d = w->dims;
   for (int l = 0; l < 4; ++l)
     if (d[l] > 1024 || (l > 0 && d[l] > 256)) return FENNOL_ERR_UNSUPPORTED;

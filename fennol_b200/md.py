@@ -208,7 +208,9 @@ class MDEngine:
         if self.trigger == "displacement":
             n += 1
         n += 1 if self.skin > 0 else 0
-        n += 1 + self.pot.mlp_launches(self.layout.ntiles) + 1 + 1  # aev fwd, mlp, energy sum, aev bwd
+        lay = self.layout
+        # aev fwd, mlp, energy sum, aev bwd
+        n += 1 + self.pot.mlp_launches(lay.ntiles, lay.rows, lay.species_mask) + 1 + 1
         return n
 
     def rebuild_launches(self) -> int:

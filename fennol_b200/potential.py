@@ -506,24 +506,19 @@ class ANIPotential:
         return max(256, int(_lib.load().fennol_mlp_workspace_bytes(self.precision, rows, self.mlp.n_models,
                                                                    self.mlp.struct)))
 
-    def mlp_launches(self, ntiles: Optional[int] = None) -> int:
-        """Kernels launched by one MLP call: the FP32 form runs 7 per
-        model, or per several models on few ``ntiles`` row tiles; the fused tcgen05 kernel (BF16 / BF16x2 on these layer sizes and the
-        FP16 forms) one, and one more for an ensemble on ``ntiles`` row tiles
-        that its CTAs share; the unfused tcgen05 path 6 per model and one sum."""
-        import os
-        if self.precision == _lib.MLP_FP32:
-            per = 1 if not ntiles else min(self.mlp.n_models, max(1, 2400 // (3 * ntiles)))
-            return 7 * -(-self.mlp.n_models // per)
-        fused = self.precision in _lib.F16_FORMS or (
-            self.precision in (_lib.MLP_BF16, _lib.MLP_BF16X2) and self.mlp.dims[0] % 256 == 0
-            and max(self.mlp.dims[1:4]) <= 256 and not os.environ.get("FENNOL_MLP_UNFUSED"))
-        if not fused:
-            return 6 * self.mlp.n_models + 1
-        if not ntiles or self.mlp.n_models == 1:
-            return 1
-        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        return 2 if ntiles % min(sms, ntiles * self.mlp.n_models) else 1
+    def mlp_launches(self, ntiles: Optional[int] = None, rows: Optional[int] = None,
+                     species_mask: Optional[int] = None, want_forces: bool = True) -> int:
+        """Kernels launched by one MLP call on ``ntiles`` row tiles
+        (``fennol_mlp_launches``); without ``ntiles``, on so many that CTAs share
+        no tile and models are evaluated one by one.  ``rows``: the layout's
+        padded rows, if more than the tiles'; ``species_mask``: the species of
+        the batch (None: every column of dE/dAEV)."""
+        if not ntiles:
+            ntiles = 8 * torch.cuda.get_device_properties(self.device).multi_processor_count
+        groups = None if species_mask is None else self.active_groups(species_mask)
+        return call("fennol_mlp_launches", self.precision, max(rows or 0, TILE * ntiles), ntiles,
+                    C_ptr(self.mlp.struct), None if groups is None else groups.ctypes.data,
+                    0 if groups is None else groups.size, int(want_forces))
 
     # --------------------------------------------------------------- launches
     def launch_forces(self, layout: BatchLayout, g: GraphBuffers, ws: Workspace, stream: int,

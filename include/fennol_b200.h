@@ -453,6 +453,13 @@ int fennol_mlp_energy_grad_groups(int precision, int rows, int ntiles, const int
                                   void* stream);
 
 /*
+ * Host only: the kernels that one fennol_mlp_energy_grad_groups call of these
+ * sizes launches (want_dx 0: with dx NULL), or FENNOL_ERR_INVALID.
+ */
+int fennol_mlp_launches(int precision, int rows, int ntiles, const fennol_mlp_weights* w,
+                        const unsigned long long* host_dx_groups, int group_words, int want_dx);
+
+/*
  * Failure handling of the fused tensor-core MLP (no counterpart in the
  * reference).  Every wait inside the kernel on a shared-memory barrier gives
  * up after a time limit: the kernel then sets the int32 error word at the

@@ -462,3 +462,40 @@ def test_fused_form_refuses_biases_off_16_bytes(cuda_device, field):
             _tile_results(pot, batch, ws)
         ctypes.memmove(ctypes.byref(pot.mlp.struct), ctypes.byref(good), ctypes.sizeof(good))
     _tile_results(pot, batch, ws)
+
+
+@pytest.mark.parametrize("precision,models", [("fp32", 1), ("fp32", 8), ("f16x3x1", 1), ("f16x3x1", 8), ("bf16x2", 3),
+                                              ("bf16x3", 2)])
+@pytest.mark.parametrize("molecules,n_side", [(0, 4), (0, 12), (30, 0), (0, 24)])
+def test_launch_count_is_what_a_call_launches(cuda_device, precision, models, molecules, n_side):
+    """The kernels of one call (the nodes of a graph it is captured in) are the ones
+    that mlp_launches counts: one or several models per launch, dX by model and
+    its sum, shared tiles and none, with and without forces."""
+    import ctypes
+
+    pot = ANIPotential(precision=precision, device=cuda_device, seed=0, n_models=models)
+    if molecules:
+        mols = molecule_batch(molecules, seed=8)
+        xyz, sp = np.concatenate([m.coordinates for m in mols]), np.concatenate([m.species for m in mols])
+        pot.energy_and_forces(xyz, sp, [m.natoms for m in mols])
+    else:
+        s = water_box(n_side, seed=1)
+        pot.energy_and_forces(s.coordinates, s.species, [s.natoms], s.cell[None])
+    layout, g, ws = next(iter(pot._cache.values()))
+    groups = pot.active_groups(layout.species_mask)
+    from fennol_b200._lib import call
+    from fennol_b200.potential import C_ptr, _ptr
+
+    for want in (True, False):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            call("fennol_mlp_energy_grad_groups", pot.precision, layout.rows, layout.ntiles,
+                 layout.t_tile_species.data_ptr(), layout.t_tile_row.data_ptr(), C_ptr(pot.mlp.struct),
+                 ws.x.data_ptr(), _ptr(ws.x_lo), groups.ctypes.data, groups.ctypes.data, groups.size,
+                 ws.e_rows.data_ptr(), ws.dx.data_ptr() if want else None, ws.mlp_ws.data_ptr(), ws.mlp_ws.numel(),
+                 torch.cuda.current_stream().cuda_stream)
+        nodes = ctypes.c_size_t()
+        rc = ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None,
+                                                              ctypes.byref(nodes))
+        assert rc == 0
+        assert nodes.value == pot.mlp_launches(layout.ntiles, layout.rows, layout.species_mask, want)
