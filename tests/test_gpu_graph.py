@@ -309,3 +309,26 @@ def test_filter_writes_each_row_once(pot, cuda_device, atoms, packed):
         got = [g2.rad_n] + [torch.where(torch.arange(cap, device=cuda_device) < g2.rad_n[:, None], t, 0)
                             for t in (g2.rad_j, g2.rad_s)]
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("molecules", [1, 3, 420])
+def test_allpairs_rows_with_and_without_cell_lists(pot, cuda_device, molecules):
+    """The all-pairs pass looks rows up only where a system of the batch has a cell
+    list: molecules alone (up to more rows than the grid has warps) get the rows
+    that they get beside a box, and the rows of the oracle."""
+    mols = molecule_batch(molecules, seed=31)
+    xyz, sp = np.concatenate([m.coordinates for m in mols]), np.concatenate([m.species for m in mols])
+    nat = [m.natoms for m in mols]
+    n = sum(nat)
+    box = water_box(8, seed=3)
+    assert molecules < 400 or n > 148 * 16 * 4
+    alone = pot.neighbor_lists(xyz, sp, nat)
+    mixed = pot.neighbor_lists(np.concatenate([xyz, box.coordinates]), np.concatenate([sp, box.species]),
+                               nat + [box.natoms], [None] * len(nat) + [box.cell])
+    assert mixed[3].plan(5.2)[2] > 0 and alone[3].plan(5.2)[2] == 0
+    assert np.array_equal(alone[2], mixed[2][:n])
+    for i in range(n):
+        k = alone[2][i]
+        assert np.array_equal(alone[0][i, :k], mixed[0][i, :k]) and np.array_equal(alone[1][i, :k], mixed[1][i, :k])
+    canon, sym = graph_fp32.canonical_from_ell(alone[0], unpack_shifts(alone[1]), alone[2])
+    assert sym and _same(canon, graph_fp32.pair_list(xyz, nat, None, None, 5.2))
