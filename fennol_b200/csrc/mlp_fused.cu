@@ -42,10 +42,11 @@
 // up to 8, whatever lies between them.
 // CELU' of layers 1-2 (needed by the backward) goes to a per-CTA scratch in
 // global memory that stays L2 resident.  Row energies are summed in model order,
-// and so is dE/dAEV (in tiles that CTAs share only up to 16 column groups, else
-// part by part), always in the same way for the same batch.  Every wait is
-// bounded (2 s); a timeout sets the error word, raises a shared abort flag that
-// ends all roles, and the CTA frees its TMEM.
+// and so is dE/dAEV, except in shared tiles where more than 16 column groups are
+// wanted and the CTAs have more than one item each: there part by part, always in
+// the same way for the same batch, but with a rounding that depends on how many
+// tiles it has.  Every wait is bounded (2 s); a timeout sets the error word, raises
+// a shared abort flag that ends all roles, and the CTA frees its TMEM.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -66,7 +67,8 @@ constexpr int kGroup = 16;                        // columns of one active-colum
 // Shared memory: a ring that every operand from global memory streams through
 // (activations live in tensor memory), an item's biases and last kernel (b1 | b2
 // | b3 | w4, 256 floats each), and per-epilogue-warp 32 x 16 dX staging tiles.
-// Ring components (an A or B tile of a chunk) start on 4 KB.
+// Ring components (an A or B tile of a chunk) start on 2 KB, the size of a dX
+// column group's weights; the swizzles repeat every 1 KB and 512 bytes.
 constexpr uint32_t kRing = 46 * 4096;
 constexpr int kBias = 256;
 constexpr uint32_t kXpose = kEpiWarps * 32 * kGroup * 4;
@@ -74,8 +76,9 @@ constexpr uint32_t kSmemMain = kRing + 4 * kBias * 4 + kXpose;
 constexpr int kChunks = 16;      // chunks in flight at most
 // L1 streams units of 32 columns (64-byte swizzle): half of a 64-column unit
 // would often be zero columns, and with all columns active two of those (96 KB
-// each with the W1 low parts) do not fit the ring: 256 molecules x 8 models 0.50
-// ms against 0.54, 98,304 atoms x 8, 8 MD steps 16.1 ms against 16.6.
+// each with the W1 low parts) do not fit the ring.  Compared when the AEV kernels
+// were slower than now: the whole call on 256 molecules x 8 models took 7 % less
+// than with 64 columns, 8 MD steps of 98,304 atoms x 8 models 3 % less.
 constexpr int kUnit = 32;
 constexpr int kMaxUnits = 4096 / kUnit, kMaxGroups = 4096 / kGroup;
 constexpr int kRunGroups = 8;    // dX column groups of one B1 run (128 columns)
@@ -230,13 +233,6 @@ __device__ __forceinline__ void celu_pair2(F2 z, F2 alpha, F2 neg_alpha, F2 k2, 
   dh = pack2(ex2(ea), ex2(eb));
   h = add2(pack2(fmaxf(a, 0.f), fmaxf(b, 0.f)), fma2(alpha, dh, neg_alpha));
 }
-__device__ __forceinline__ F2 dcelu2(F2 z, F2 k2) {
-  float a, b;
-  unpack2(z, a, b);
-  float ea, eb;
-  unpack2(mul2(pack2(fminf(a, 0.f), fminf(b, 0.f)), k2), ea, eb);
-  return pack2(ex2(ea), ex2(eb));
-}
 
 // Bounded wait that also gives up when another role has aborted.
 // Threads sleep in mbarrier.try_wait (woken when the phase completes) instead
@@ -257,8 +253,8 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   }
 }
 
-// 16 columns of a row as 16-bit pairs: w[0..7] the high parts, w[8..15] the
-// residuals (BF16, or FP16 when F16); one paired conversion per two columns.
+// Two columns of a row as packed 16-bit values: the high parts and, with_lo, the
+// residuals (BF16, or FP16 when F16), each by one paired conversion.
 template <bool F16>
 __device__ __forceinline__ void split_pair(F2 v, bool with_lo, uint32_t& hi, uint32_t& lo) {
   float a, b;

@@ -108,30 +108,13 @@ __device__ __forceinline__ void tma_load_2d_hint(const CUtensorMap* map, uint64_
       : "memory");
 }
 
-// Shared -> global bulk tensor copies (bulk-group completion): a plain store
-// and an in-L2 FP32 add.  The source tile is laid out as the map's swizzle says.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"((uint64_t)map), "r"(smem_u32(src)), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, const void* src, int x, int y) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"((uint64_t)map), "r"(smem_u32(src)), "r"(x), "r"(y)
-               : "memory");
-}
+// Shared -> global bulk tensor store (bulk-group completion).  The source tile is
+// laid out as the map's swizzle says.
 __device__ __forceinline__ void tma_store_2d_hint(const CUtensorMap* map, const void* src, int x, int y,
                                                   uint64_t pol) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;"
                ::"l"((uint64_t)map), "r"(smem_u32(src)), "r"(x), "r"(y), "l"(pol)
                : "memory");
-}
-__device__ __forceinline__ void tma_add_2d_hint(const CUtensorMap* map, const void* src, int x, int y,
-                                                uint64_t pol) {
-  asm volatile(
-      "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;"
-      ::"l"((uint64_t)map), "r"(smem_u32(src)), "r"(x), "r"(y), "l"(pol)
-      : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // the sources of this thread's bulk copies may be overwritten
