@@ -462,6 +462,9 @@ class ServingEngine:
         self.bytes_per_atom = d0 * (act + 4) + 8 * 128 + 256
         self.bytes_per_atom_md = self.bytes_per_atom + 8 * 96 + 128
         self._mlp_bytes: Dict[int, int] = {}
+        # the scratch of a full lane: what has room for it needs no closer look
+        self._full_atoms = max(max_ef_atoms, max_md_atoms)
+        self._full_bytes = self.batch_bytes(self._full_atoms, 0)
         self.bytes_in_flight = 0
         self.results: List[ServeResult] = []
         self.ef = _EFLane(self)
@@ -476,6 +479,13 @@ class ServingEngine:
             self._mlp_bytes[tiles] = self.pot.mlp_workspace_bytes(TILE * tiles)
         return per_atom * atoms + self._mlp_bytes[tiles]
 
+    def _fits(self, used: int, atoms: int, per_atom: int) -> bool:
+        """A batch beside ``used`` bytes stays within the budget."""
+        room = self.budget - used - per_atom * atoms
+        if atoms <= self._full_atoms and room >= self._full_bytes:
+            return True
+        return room >= self.batch_bytes(atoms, 0)
+
     def _md_admits(self, running: int, pop: bool) -> List[tuple]:
         """Ready MD requests, in order, that fit beside ``running`` atoms in
         the MD lane's atom limit and in the HBM budget (the bytes of the
@@ -486,7 +496,7 @@ class ServingEngine:
         admit, atoms = [], running
         for item in list(md.ready):
             n_new = item[0].natoms
-            fits = n_new <= room and other + self.batch_bytes(atoms + n_new, self.bytes_per_atom_md) <= self.budget
+            fits = n_new <= room and self._fits(other, atoms + n_new, self.bytes_per_atom_md)
             if not fits and (admit or running or other):
                 break
             admit.append(item)
@@ -502,8 +512,7 @@ class ServingEngine:
             r = queue[0]
             if out and atoms + r.natoms > max_atoms:
                 break
-            if (out or self.bytes_in_flight) and \
-                    self.bytes_in_flight + self.batch_bytes(atoms + r.natoms, per_atom) > self.budget:
+            if (out or self.bytes_in_flight) and not self._fits(self.bytes_in_flight, atoms + r.natoms, per_atom):
                 break
             out.append(queue.popleft())
             atoms += r.natoms
